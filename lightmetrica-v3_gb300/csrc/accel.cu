@@ -62,8 +62,8 @@ __device__ inline float refine_hit_t(const float4 ra, const float4 rb, const flo
     return lmgpu_ht::hit_t(o, d, p1, e1, e2);
 }
 
-// rays: 2 float4 per ray (o, tmin) (d, tmax). refill > 0: block b of G takes the groups of 32
-// consecutive rays b, b + G, b + 2G, ... and its warps fetch from them dynamically through a
+// rays: 2 float4 per ray (o, tmin) (d, tmax). refill > 0: block b of G takes the groups of
+// 2^group_log2 consecutive rays b, b + G, b + 2G, ... and its warps fetch from them dynamically through a
 // shared-memory counter (no state outside the launch, so calls on several streams may overlap).
 // Interleaving the groups gives every block a sample of the whole batch: with one contiguous
 // chunk per block, rays in caller order (camera rays, bounces sorted by origin or direction) left
@@ -72,12 +72,11 @@ __device__ inline float refine_hit_t(const float4 ra, const float4 rb, const flo
 template <bool kAnyHit, bool kTwoLevel>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(Bvh8 bvh, const float4* __restrict__ rays, int64_t n,
                                                             lmgpu_hit* __restrict__ hits, uint8_t* __restrict__ occluded,
-                                                            int* __restrict__ err, int refill) {
-    extern __shared__ uint32_t smem[];
+                                                            int* __restrict__ err, int refill, int group_log2) {
+    extern __shared__ uint2 smem[];
     __shared__ int s_fetch;
     const int stride = blockDim.x;
-    uint32_t* sb = smem + threadIdx.x;
-    uint32_t* sbits = smem + stride * bvh.depth + threadIdx.x;
+    uint2* stk = smem + threadIdx.x;
     int lerr = 0;
     auto store = [&](int64_t i, const TraceHit& h) {
         if (kAnyHit) {
@@ -93,26 +92,26 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(Bvh8 bvh, const flo
     };
     if (refill > 0) {
         const int64_t G = gridDim.x, blk = blockIdx.x;
-        const int64_t ngroups = (n + 31) / 32;
+        const int64_t gs = int64_t(1) << group_log2, ngroups = (n + gs - 1) >> group_log2;
         const int64_t mine = blk < ngroups ? (ngroups - 1 - blk) / G + 1 : 0;
         // only the batch's last group can be short, and it is this block's last one if it is ours
-        int64_t count = mine * 32;
-        if (mine > 0 && blk + (mine - 1) * G == ngroups - 1) count -= ngroups * 32 - n;
-        auto ray_of = [&](int k) { return (blk + int64_t(k >> 5) * G) * 32 + (k & 31); };
+        int64_t count = mine << group_log2;
+        if (mine > 0 && blk + (mine - 1) * G == ngroups - 1) count -= ngroups * gs - n;
+        auto ray_of = [&](int k) { return ((blk + int64_t(k >> group_log2) * G) << group_log2) + (k & int(gs - 1)); };
         if (threadIdx.x == 0) s_fetch = 0;
         __syncthreads();
         fetch_loop<kAnyHit, false, kTwoLevel>(
-            int(count), Fetch{&s_fetch, nullptr, refill}, bvh, sb, sbits, stride, &lerr,
-            [&](int k, Trav& s, Bvh8&) {
+            int(count), int(blockDim.x / 32), Fetch{&s_fetch, nullptr, refill}, stk, stride, &lerr,
+            [&](int k, Trav& s) {
                 const int64_t i = ray_of(k);
                 const float4 a = rays[2 * i], b = rays[2 * i + 1];
                 trav_init(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w);
             },
-            [&](int k, const Trav& s) { store(ray_of(k), s.best); });
+            [&](int) { return bvh; }, [&](int k, const Trav& s) { store(ray_of(k), s.best); });
     } else {
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
             const float4 a = rays[2 * i], b = rays[2 * i + 1];
-            store(i, trace_bvh8<kAnyHit, false, kTwoLevel>(bvh, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, sb, sbits, stride,
+            store(i, trace_bvh8<kAnyHit, false, kTwoLevel>(bvh, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, stk, stride,
                                                 nullptr, nullptr, &lerr));
         }
     }
@@ -137,16 +136,15 @@ __global__ void __launch_bounds__(256) k_refine_hits(const float4* __restrict__ 
 template <bool kAnyHit, bool kTwoLevel>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_count(Bvh8 bvh, const float4* __restrict__ rays, int64_t n,
                                                             int sample, unsigned long long* sums, int* err) {
-    extern __shared__ uint32_t smem[];
+    extern __shared__ uint2 smem[];
     const int stride = blockDim.x;
-    uint32_t* sb = smem + threadIdx.x;
-    uint32_t* sbits = smem + stride * bvh.depth + threadIdx.x;
+    uint2* stk = smem + threadIdx.x;
     int lerr = 0;
     uint32_t nodes = 0, tris = 0, cnt = 0;
     for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j * sample < n; j += int64_t(gridDim.x) * blockDim.x) {
         const int64_t i = j * sample;
         const float4 a = rays[2 * i], b = rays[2 * i + 1];
-        trace_bvh8<kAnyHit, true, kTwoLevel>(bvh, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, sb, sbits, stride, &nodes, &tris,
+        trace_bvh8<kAnyHit, true, kTwoLevel>(bvh, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, stk, stride, &nodes, &tris,
                                   &lerr);
         cnt++;
     }
@@ -157,15 +155,11 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_count(Bvh8 bvh, const flo
 }
 
 template <typename K>
-int trace_grid(K kernel, size_t smem, int64_t n) {
+int resident_blocks(K kernel, size_t smem) {
     if (smem > 48 * 1024) LMGPU_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     int per_sm = 0;
     LMGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTraceBlock, smem));
-    per_sm = per_sm < 1 ? 1 : per_sm;
-    const int64_t need = (n + kTraceBlock - 1) / kTraceBlock;
-    int64_t g = int64_t(per_sm) * current_device().num_sms;
-    if (need < g) g = need;
-    return int(g < 1 ? 1 : g);
+    return (per_sm < 1 ? 1 : per_sm) * current_device().num_sms;
 }
 
 Bvh8 device_view(const lmgpu_accel* a) {
@@ -195,9 +189,15 @@ void launch_trace(const lmgpu_accel* a, const void* d_rays, int64_t n, void* d_h
     const Bvh8 b = device_view(a);
     const size_t smem = trace_smem(a);
     auto run = [&](auto kernel) {
-        const int g = trace_grid(kernel, smem, n);
+        // Rays per group: 32, or fewer when the batch has fewer rays than the chip has lanes, so that
+        // they spread over all warps; down to the four rays of a cooperative warp.
+        const int warps = kTraceBlock / 32, gmax = resident_blocks(kernel, smem);
+        int gl = 2;
+        while (gl < 5 && ((n + (int64_t(1) << gl) - 1) >> gl) > int64_t(gmax) * warps) gl++;
+        const int64_t groups = (n + (int64_t(1) << gl) - 1) >> gl;
+        const int g = int(std::min<int64_t>(gmax, tuning().trace_refill > 0 ? (groups + warps - 1) / warps : (n + kTraceBlock - 1) / kTraceBlock));
         kernel<<<g, kTraceBlock, smem, st>>>(b, static_cast<const float4*>(d_rays), n, static_cast<lmgpu_hit*>(d_hits), d_occ,
-                                             d_err, tuning().trace_refill);
+                                             d_err, tuning().trace_refill, gl);
     };
     const bool two = a->num_instances > 0;
     if (d_occ) two ? run(k_trace_batch<true, true>) : run(k_trace_batch<true, false>);
@@ -674,7 +674,7 @@ int lmgpu_accel_trace_counts(lmgpu_accel* accel, const void* d_rays, int64_t n, 
         const size_t smem = trace_smem(accel);
         const int64_t m = (n + sample - 1) / sample;
         auto run = [&](auto kernel) {
-            const int g = trace_grid(kernel, smem, m);
+            const int g = int(std::min<int64_t>(resident_blocks(kernel, smem), (m + kTraceBlock - 1) / kTraceBlock));
             kernel<<<g, kTraceBlock, smem>>>(b, static_cast<const float4*>(d_rays), n, sample, sums.as<unsigned long long>(),
                                              accel->err.as<int>());
         };

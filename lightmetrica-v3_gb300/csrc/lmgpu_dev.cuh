@@ -118,19 +118,8 @@ __device__ inline bool tri_test(f3 o, f3 d, f3 p1, f3 e1, f3 e2, float tl, float
     return true;
 }
 
-__device__ inline uint32_t byte_of(uint32_t w, int k) { return (w >> (8 * k)) & 0xffu; }
-
 // Three-input min / max (one instruction each on sm_100 and later; exact, like the two-input
 // forms, so the slab test's result does not change).
-#ifndef LMGPU_TRAV_SPLIT
-// persistent traversal steps: 0 = a node and all its entered leaf triangles per step (trav_step);
-// 1 = a node or one triangle per step (trav_step_split); 2 = as 1, and a closest-hit step that
-// tests a node's last pending triangle goes on to the next node (measured on the displaced-sphere
-// frame: extension 70.7 -> 64.5 ms, shadow 27.5 -> 27.2 ms per 64-spp frame)
-#define LMGPU_TRAV_SPLIT 2
-#endif
-
-#ifndef LMGPU_NO_MINMAX3
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
@@ -141,17 +130,24 @@ __device__ __forceinline__ float fmin3(float a, float b, float c) {
     asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-#else
-__device__ __forceinline__ float fmax3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
-__device__ __forceinline__ float fmin3(float a, float b, float c) { return fminf(fminf(a, b), c); }
-#endif
 
-// Permutes the 8 slot bits of `m` so that bit (s ^ oct) holds slot s.
-__device__ inline uint32_t oct_permute(uint32_t m, uint32_t oct) {
-    if (oct & 1u) m = ((m & 0x55u) << 1) | ((m >> 1) & 0x55u);
-    if (oct & 2u) m = ((m & 0x33u) << 2) | ((m >> 2) & 0x33u);
-    if (oct & 4u) m = ((m & 0x0fu) << 4) | ((m >> 4) & 0x0fu);
-    return m;
+// Two fp32 FMAs in one instruction (sm_100 and later), each rounded as fmaf rounds it.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t a, uint32_t b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ float2 fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    float2 v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
+    return v;
 }
 
 // Ray traversal of the 8-wide BVH. Closest hit: the smallest t over every triangle whose test
@@ -159,12 +155,11 @@ __device__ inline uint32_t oct_permute(uint32_t m, uint32_t oct) {
 // (`any_hit`): ends at the first accepted triangle. The per-thread stack of sibling groups
 // lives in shared memory: stk[i * stride] for i < bvh.depth. Child boxes carry a margin of one
 // quantum and the slab comparison widens by 2^-18 relative, which bounds the rounding of the
-// one-FMA slab distances (see the node visit below), so no triangle the exact test would accept
-// is culled.
+// one-FMA slab distances (see Slabs), so no triangle the exact test would accept is culled.
 //
-// The traversal is a resumable state (Trav) advanced one node visit at a time by trav_step, so
-// a persistent kernel can interleave rays on a lane (dynamic ray fetch); trace_bvh8 runs one ray
-// to the end. Either way a ray's visits, tests and result are the same.
+// The traversal is a resumable state (Trav) advanced one step at a time, so a persistent kernel
+// can interleave rays on a lane (dynamic ray fetch); trace_bvh8 runs one ray to the end. Either
+// way a ray's visits, tests and result are the same.
 //
 // Two-level trees (kTwoLevel): a top-level child whose node carries the instance marker
 // (exponent byte 0xFF) stands for one instance. Visiting it saves the world ray, moves the ray
@@ -178,18 +173,17 @@ struct Trav {
     float tmin;
     uint32_t oct;
     int sp;
-    uint32_t node;
+    uint32_t node;  // the node to visit next; kNoNode: none is left
     uint32_t nvis, ntri;
     TraceHit best;
     // two-level only (never read, so never allocated, in single-level code)
     f3 wo, wd;
     int inst_sp;
     int32_t id_base;
-#if LMGPU_TRAV_SPLIT
     // split steps: the entered leaf triangles of the last node, tested one per step
     uint32_t tri_base, tri_mask;
-#endif
 };
+constexpr uint32_t kNoNode = 0xffffffffu;
 
 __device__ inline void trav_set_ray(Trav& s, f3 o, f3 d) {
     s.o = o;
@@ -215,9 +209,158 @@ __device__ inline void trav_init(Trav& s, f3 o, f3 d, float tmin, float tmax) {
     s.ntri = 0;
     s.inst_sp = -1;
     s.id_base = 0;
-#if LMGPU_TRAV_SPLIT
     s.tri_mask = 0u;
-#endif
+}
+
+// Slab distances of one node for one ray, with one FMA per plane. Plane q of an axis lies at
+// p + q*s; with a = s*inv and b = (p - o)*inv, t = q*a + b. The byte is unpacked straight into
+// the float X = 2^23 + 256*q (one byte permute), so t = fma(X, a/256, b - 2^15*a): the large
+// offset cancels exactly inside the FMA. Error: about 5 ulp relative plus 0.003 quanta absolute;
+// the builder leaves one quantum of margin around every child box and the comparison widens the
+// far side by 2^-18 relative (kWiden), so the test never culls a box the exact ray enters.
+struct Slabs {
+    float ax, ay, az, bx, by, bz;
+};
+constexpr float kWiden = 1.0000038f;
+__device__ __forceinline__ Slabs node_slabs(const uint4& w0, const Trav& s) {
+    const float ax = __uint_as_float((w0.w & 0xffu) << 23) * s.inv.x;
+    const float ay = __uint_as_float(((w0.w >> 8) & 0xffu) << 23) * s.inv.y;
+    const float az = __uint_as_float(((w0.w >> 16) & 0xffu) << 23) * s.inv.z;
+    const float bx = (__uint_as_float(w0.x) - s.o.x) * s.inv.x;
+    const float by = (__uint_as_float(w0.y) - s.o.y) * s.inv.y;
+    const float bz = (__uint_as_float(w0.z) - s.o.z) * s.inv.z;
+    return Slabs{ax * 0.00390625f, ay * 0.00390625f, az * 0.00390625f,
+                 fmaf(-32768.0f, ax, bx), fmaf(-32768.0f, ay, by), fmaf(-32768.0f, az, bz)};
+}
+
+// The children of a node whose boxes the ray enters in [tmin, best.t], one bit per slot (plane
+// words: qlo x y z, then qhi x y z, two words each).
+__device__ __forceinline__ uint32_t node_children(const uint4& w0, const uint4& w2, const uint4& w3, const uint4& w4, const Trav& s) {
+    const Slabs S = node_slabs(w0, s);
+    const uint64_t ax2 = pack2(S.ax, S.ax), ay2 = pack2(S.ay, S.ay), az2 = pack2(S.az, S.az);
+    const uint64_t bx2 = pack2(S.bx, S.bx), by2 = pack2(S.by, S.by), bz2 = pack2(S.bz, S.bz);
+    // near/far plane bytes per axis, chosen by the ray's octant
+    const bool ox = s.oct & 1u, oy = s.oct & 2u, oz = s.oct & 4u;
+    const uint32_t nx0 = ox ? w3.z : w2.x, nx1 = ox ? w3.w : w2.y, fx0 = ox ? w2.x : w3.z, fx1 = ox ? w2.y : w3.w;
+    const uint32_t ny0 = oy ? w4.x : w2.z, ny1 = oy ? w4.y : w2.w, fy0 = oy ? w2.z : w4.x, fy1 = oy ? w2.w : w4.y;
+    const uint32_t nz0 = oz ? w4.z : w3.x, nz1 = oz ? w4.w : w3.y, fz0 = oz ? w3.x : w4.z, fz1 = oz ? w3.y : w4.w;
+    // The trace kernels are bound by instruction issue (70-79 % of the slots, the nodes in L1 and L2),
+    // a node's 48 planes being most of it: two slots per instruction (fma.f32x2), and the comparison
+    // near <= far * kWiden as the sign of far * kWiden - near shifted into the mask, slot 7 first
+    // (2^20 diffuse bounces in a soup of 60k triangles: 781 -> 710 us; one FMA per plane 2 % and
+    // compares with set bits 3 % slower). Empty slots hold inverted boxes
+    // (qlo = 255, qhi = 0) that no ray enters; one accepted through rounding is a leaf of zero
+    // triangles.
+    uint32_t miss = 0u;
+#pragma unroll
+    for (int k = 6; k >= 0; k -= 2) {
+        const uint32_t s0 = 0x5404u | (uint32_t(k & 3) << 4), s1 = s0 + 0x10u;  // bytes: 00, q, 00, 4B
+        auto planes = [&](uint32_t w, uint64_t a, uint64_t b) {
+            return fma2(pack2(__byte_perm(w, 0x4B00u, s0), __byte_perm(w, 0x4B00u, s1)), a, b);
+        };
+        const float2 xn = planes(k < 4 ? nx0 : nx1, ax2, bx2), xf = planes(k < 4 ? fx0 : fx1, ax2, bx2);
+        const float2 yn = planes(k < 4 ? ny0 : ny1, ay2, by2), yf = planes(k < 4 ? fy0 : fy1, ay2, by2);
+        const float2 zn = planes(k < 4 ? nz0 : nz1, az2, bz2), zf = planes(k < 4 ? fz0 : fz1, az2, bz2);
+        const float n0 = fmax3(xn.x, yn.x, fmaxf(zn.x, s.tmin)), n1 = fmax3(xn.y, yn.y, fmaxf(zn.y, s.tmin));
+        const float f0 = fmin3(xf.x, yf.x, fminf(zf.x, s.best.t)), f1 = fmin3(xf.y, yf.y, fminf(zf.y, s.best.t));
+        miss = __funnelshift_l(__float_as_uint(fmaf(f1, kWiden, -n1)), miss, 1);
+        miss = __funnelshift_l(__float_as_uint(fmaf(f0, kWiden, -n0)), miss, 1);
+    }
+    return ~miss & 0xffu;
+}
+
+// The triangles of a leaf child, from its meta byte (the low byte of `meta`): count << 5 | offset.
+__device__ __forceinline__ uint32_t leaf_bits(uint32_t meta) {
+    uint32_t m;
+    asm("bmsk.clamp.b32 %0, %1, %2;" : "=r"(m) : "r"(meta & 31u), "r"((meta >> 5) & 7u));
+    return m;
+}
+
+// The triangles of the entered leaf children, one bit per triangle after the node's first one.
+__device__ __forceinline__ uint32_t leaf_triangles(const uint4& w1, uint32_t leaves) {
+    uint32_t tmask = 0u;
+    while (leaves) {
+        const int k = __ffs(leaves) - 1;
+        leaves &= leaves - 1;
+        tmask |= leaf_bits(__byte_perm(w1.z, w1.w, uint32_t(k)));
+    }
+    return tmask;
+}
+
+// Tests the first triangle of s.tri_mask. Any hit: true if the ray hits it.
+template <bool kAnyHit, bool kCount, bool kTwoLevel>
+__device__ __forceinline__ bool trav_test_tri(const Bvh8& bvh, Trav& s) {
+    const int j = __ffs(s.tri_mask) - 1;
+    s.tri_mask &= s.tri_mask - 1u;
+    const float4* tp = bvh.tris + size_t(s.tri_base + uint32_t(j)) * 3;
+    const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+    if (kCount) s.ntri++;
+    float t, u, v;
+    if (tri_test(s.o, s.d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), s.tmin, s.best.t, t, u, v)) {
+        const int32_t id = (kTwoLevel ? s.id_base : 0) + int32_t(__float_as_uint(c.y));
+        if (kAnyHit) {
+            s.best = TraceHit{t, u, v, id};
+            return true;
+        }
+        if (t < s.best.t || s.best.id < 0 || id < s.best.id) s.best = TraceHit{t, u, v, id};
+    }
+    return false;
+}
+
+// The instance pseudo-node (w0, w1): the ray continues in the instance's frame at its BLAS root.
+__device__ __forceinline__ void trav_enter_instance(const Bvh8& bvh, Trav& s, const uint4& w1) {
+    const float4* ip = bvh.inst + size_t(w1.x) * 4;
+    const float4 r0 = __ldg(ip), r1 = __ldg(ip + 1), r2 = __ldg(ip + 2);
+    const uint4 m = __ldg(reinterpret_cast<const uint4*>(ip + 3));
+    s.wo = s.o;
+    s.wd = s.d;
+    const f3 lo = {r0.x * s.o.x + r0.y * s.o.y + r0.z * s.o.z + r0.w, r1.x * s.o.x + r1.y * s.o.y + r1.z * s.o.z + r1.w,
+                   r2.x * s.o.x + r2.y * s.o.y + r2.z * s.o.z + r2.w};
+    const f3 ld = {r0.x * s.d.x + r0.y * s.d.y + r0.z * s.d.z, r1.x * s.d.x + r1.y * s.d.y + r1.z * s.d.z,
+                   r2.x * s.d.x + r2.y * s.d.y + r2.z * s.d.z};
+    trav_set_ray(s, lo, ld);
+    s.inst_sp = s.sp;
+    s.id_base = int32_t(m.y);
+    s.node = m.x;
+}
+
+// Chooses s.node: the nearest of the entered inner children `inner` (slots of the node whose
+// children start at `base`, with child mask `imask`), else of the sibling group on top of the
+// stack, else kNoNode. False on a stack overflow. `write`: this lane stores the stack entry.
+template <bool kTwoLevel>
+__device__ __forceinline__ bool trav_next(const Bvh8& bvh, Trav& s, uint32_t base, uint32_t imask, uint32_t inner, uint2* stk,
+                                          int stride, bool write = true) {
+    if (inner == 0u) {
+        if (kTwoLevel && s.sp == s.inst_sp) {  // the instance is done: back to the world ray
+            trav_set_ray(s, s.wo, s.wd);
+            s.inst_sp = -1;
+            s.id_base = 0;
+        }
+        if (s.sp == 0) {
+            s.node = kNoNode;
+            return true;
+        }
+        s.sp--;
+        const uint2 g = stk[s.sp * stride];
+        base = g.x;
+        imask = g.y >> 8;
+        inner = g.y & 0xffu;
+    }
+    // nearest first by octant order: the slot with the smallest slot ^ octant, as a one-bit mask
+    uint32_t first = inner, part = first & ((s.oct & 4u) ? 0xf0u : 0x0fu);
+    first = part ? part : first;
+    part = first & ((s.oct & 2u) ? 0xccu : 0x33u);
+    first = part ? part : first;
+    part = first & ((s.oct & 1u) ? 0xaau : 0x55u);
+    first = part ? part : first;
+    s.node = base + __popc(imask & (first - 1u));
+    inner ^= first;
+    if (inner != 0u) {
+        if (s.sp >= bvh.depth) return false;
+        if (write) stk[s.sp * stride] = make_uint2(base, (imask << 8) | inner);
+        s.sp++;
+    }
+    return true;
 }
 
 // Visits s.node (testing the triangles of every leaf child the ray enters) and moves to the next
@@ -225,280 +368,60 @@ __device__ inline void trav_init(Trav& s, f3 o, f3 d, float tmin, float tmax) {
 // ends) on a stack overflow (1) or a visit count above the node count (2), which only a corrupt
 // BVH can cause.
 template <bool kAnyHit, bool kCount, bool kTwoLevel = false>
-__device__ __forceinline__ bool trav_step(const Bvh8& bvh, Trav& s, uint32_t* stk_base, uint32_t* stk_bits, int stride,
-                                          int* err) {
+__device__ __forceinline__ bool trav_step(const Bvh8& bvh, Trav& s, uint2* stk, int stride, int* err) {
     if (s.node >= bvh.num_nodes || s.nvis >= bvh.max_visits) { *err = 2; return true; }
     const uint4* np = bvh.nodes + size_t(s.node) * 5;
     const uint4 w0 = __ldg(np), w1 = __ldg(np + 1);
     s.nvis++;
     if (kTwoLevel && (w0.w & 0xffu) == 0xffu) {
-        // instance pseudo-node: continue in the instance's frame at its BLAS root
-        const float4* ip = bvh.inst + size_t(w1.x) * 4;
-        const float4 r0 = __ldg(ip), r1 = __ldg(ip + 1), r2 = __ldg(ip + 2);
-        const uint4 m = __ldg(reinterpret_cast<const uint4*>(ip + 3));
-        s.wo = s.o;
-        s.wd = s.d;
-        const f3 lo = {r0.x * s.o.x + r0.y * s.o.y + r0.z * s.o.z + r0.w, r1.x * s.o.x + r1.y * s.o.y + r1.z * s.o.z + r1.w,
-                       r2.x * s.o.x + r2.y * s.o.y + r2.z * s.o.z + r2.w};
-        const f3 ld = {r0.x * s.d.x + r0.y * s.d.y + r0.z * s.d.z, r1.x * s.d.x + r1.y * s.d.y + r1.z * s.d.z,
-                       r2.x * s.d.x + r2.y * s.d.y + r2.z * s.d.z};
-        trav_set_ray(s, lo, ld);
-        s.inst_sp = s.sp;
-        s.id_base = int32_t(m.y);
-        s.node = m.x;
+        trav_enter_instance(bvh, s, w1);
         return false;
     }
     const uint4 w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
-    const uint32_t oct = s.oct;
-    // Slab distances with one FMA per plane. Plane q of an axis lies at p + q*s; with
-    // a = s*inv and b = (p - o)*inv, t = q*a + b. The byte is unpacked straight into the float
-    // X = 2^23 + 256*q (one byte permute), so t = fma(X, a/256, b - 2^15*a): the large offset
-    // cancels exactly inside the FMA. Error: about 5 ulp relative plus 0.003 quanta absolute;
-    // the builder leaves one quantum of margin around every child box and the comparison
-    // widens by 2^-18 relative, so the test never culls a box the exact ray enters.
-    const float sx = __uint_as_float((w0.w & 0xffu) << 23);
-    const float sy = __uint_as_float(((w0.w >> 8) & 0xffu) << 23);
-    const float sz = __uint_as_float(((w0.w >> 16) & 0xffu) << 23);
-    const uint32_t imask = w0.w >> 24;
-    const float ax = sx * s.inv.x, ay = sy * s.inv.y, az = sz * s.inv.z;
-    const float bx = (__uint_as_float(w0.x) - s.o.x) * s.inv.x;
-    const float by = (__uint_as_float(w0.y) - s.o.y) * s.inv.y;
-    const float bz = (__uint_as_float(w0.z) - s.o.z) * s.inv.z;
-    const float ax8 = ax * 0.00390625f, ay8 = ay * 0.00390625f, az8 = az * 0.00390625f;
-    const float bx8 = fmaf(-32768.0f, ax, bx), by8 = fmaf(-32768.0f, ay, by), bz8 = fmaf(-32768.0f, az, bz);
-    // near/far plane bytes per axis, chosen by the ray's octant
-    const uint32_t lx0 = w2.x, lx1 = w2.y, ly0 = w2.z, ly1 = w2.w, lz0 = w3.x, lz1 = w3.y;
-    const uint32_t hx0 = w3.z, hx1 = w3.w, hy0 = w4.x, hy1 = w4.y, hz0 = w4.z, hz1 = w4.w;
-    const uint32_t nx0 = (oct & 1u) ? hx0 : lx0, nx1 = (oct & 1u) ? hx1 : lx1;
-    const uint32_t fx0 = (oct & 1u) ? lx0 : hx0, fx1 = (oct & 1u) ? lx1 : hx1;
-    const uint32_t ny0 = (oct & 2u) ? hy0 : ly0, ny1 = (oct & 2u) ? hy1 : ly1;
-    const uint32_t fy0 = (oct & 2u) ? ly0 : hy0, fy1 = (oct & 2u) ? ly1 : hy1;
-    const uint32_t nz0 = (oct & 4u) ? hz0 : lz0, nz1 = (oct & 4u) ? hz1 : lz1;
-    const uint32_t fz0 = (oct & 4u) ? lz0 : hz0, fz1 = (oct & 4u) ? lz1 : hz1;
-    uint32_t hitmask = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const uint32_t sel = 0x5404u | (uint32_t(k & 3) << 4);  // bytes: 00, q, 00, 4B
-        const float qnx = __uint_as_float(__byte_perm(k < 4 ? nx0 : nx1, 0x4B00u, sel));
-        const float qfx = __uint_as_float(__byte_perm(k < 4 ? fx0 : fx1, 0x4B00u, sel));
-        const float qny = __uint_as_float(__byte_perm(k < 4 ? ny0 : ny1, 0x4B00u, sel));
-        const float qfy = __uint_as_float(__byte_perm(k < 4 ? fy0 : fy1, 0x4B00u, sel));
-        const float qnz = __uint_as_float(__byte_perm(k < 4 ? nz0 : nz1, 0x4B00u, sel));
-        const float qfz = __uint_as_float(__byte_perm(k < 4 ? fz0 : fz1, 0x4B00u, sel));
-        const float tn = fmax3(fmaf(qnx, ax8, bx8), fmaf(qny, ay8, by8), fmaxf(fmaf(qnz, az8, bz8), s.tmin));
-        const float tf0 = fmin3(fmaf(qfx, ax8, bx8), fmaf(qfy, ay8, by8), fminf(fmaf(qfz, az8, bz8), s.best.t));
-        // Widening the far side by 2^-18 covers the relative error of both sides. Empty slots
-        // hold inverted boxes (qlo = 255, qhi = 0) that no ray enters; one accepted through
-        // rounding is a leaf of zero triangles.
-        if (tn <= tf0 * 1.0000038f) hitmask |= 1u << k;
-    }
-    // ---- leaf children: test their triangles now -----------------------------------------------
-    uint32_t leaves = hitmask & ~imask;
-    while (leaves) {
-        const int k = __ffs(leaves) - 1;
-        leaves &= leaves - 1;
-        const uint32_t meta = byte_of(k < 4 ? w1.z : w1.w, k & 3);
-        const uint32_t cnt = meta >> 5, off = meta & 31u;
-        for (uint32_t j = 0; j < cnt; j++) {
-            const float4* tp = bvh.tris + size_t(w1.y + off + j) * 3;
-            const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-            if (kCount) s.ntri++;
-            float t, u, v;
-            if (tri_test(s.o, s.d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), s.tmin, s.best.t, t, u, v)) {
-                const int32_t id = (kTwoLevel ? s.id_base : 0) + int32_t(__float_as_uint(c.y));
-                if (kAnyHit) {
-                    s.best = TraceHit{t, u, v, id};
-                    return true;
-                }
-                if (t < s.best.t || s.best.id < 0 || id < s.best.id) s.best = TraceHit{t, u, v, id};
-            }
-        }
-    }
-    // ---- next node: nearest-first by octant order ----------------------------------------------
-    uint32_t inner = oct_permute(hitmask & imask, oct);
-    uint32_t g_base = w1.x, g_imask = imask;
-    if (inner == 0u) {
-        if (kTwoLevel && s.sp == s.inst_sp) {  // the instance is done: back to the world ray
-            trav_set_ray(s, s.wo, s.wd);
-            s.inst_sp = -1;
-            s.id_base = 0;
-        }
-        if (s.sp == 0) return true;
-        s.sp--;
-        g_base = stk_base[s.sp * stride];
-        const uint32_t bits = stk_bits[s.sp * stride];
-        g_imask = bits >> 8;
-        inner = bits & 0xffu;
-    }
-    const int k = __ffs(inner) - 1;
-    inner &= inner - 1;
-    const uint32_t slot = uint32_t(k) ^ s.oct;
-    s.node = g_base + __popc(g_imask & ((1u << slot) - 1u));
-    if (inner != 0u) {
-        if (s.sp >= bvh.depth) { *err = 1; return true; }
-        stk_base[s.sp * stride] = g_base;
-        stk_bits[s.sp * stride] = (g_imask << 8) | inner;
-        s.sp++;
-    }
-    return false;
+    const uint32_t hit = node_children(w0, w2, w3, w4, s), imask = w0.w >> 24;
+    s.tri_base = w1.y;
+    s.tri_mask = leaf_triangles(w1, hit & ~imask);
+    while (s.tri_mask)
+        if (trav_test_tri<kAnyHit, kCount, kTwoLevel>(bvh, s)) return true;
+    if (!trav_next<kTwoLevel>(bvh, s, w1.x, imask, hit & imask, stk, stride)) { *err = 1; return true; }
+    return s.node == kNoNode;
 }
 
-#if LMGPU_TRAV_SPLIT
 // trav_step with finer steps (after the triangle-postponing traversal of Ylitie et al., HPG 2017):
 // a node step records the triangles of the leaf children the ray enters as a mask; each later
 // step tests one of them; the next node is visited once the mask is empty. The order of tests is
 // trav_step's, so the result is the same; a warp's lanes now diverge between a node step and
-// one triangle test instead of waiting for the lane with the most triangles.
-template <bool kAnyHit, bool kCount, bool kTwoLevel = false>
-__device__ __forceinline__ bool trav_step_split(const Bvh8& bvh, Trav& s, uint32_t* stk_base, uint32_t* stk_bits, int stride,
-                                                int* err) {
+// one triangle test instead of waiting for the lane with the most triangles. Single-level trees.
+template <bool kAnyHit, bool kCount>
+__device__ __forceinline__ bool trav_step_split(const Bvh8& bvh, Trav& s, uint2* stk, int stride, int* err) {
     if (s.tri_mask) {
-        const int j = __ffs(s.tri_mask) - 1;
-        s.tri_mask &= s.tri_mask - 1u;
-        const float4* tp = bvh.tris + size_t(s.tri_base + uint32_t(j)) * 3;
-        const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-        if (kCount) s.ntri++;
-        float t, u, v;
-        if (tri_test(s.o, s.d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), s.tmin, s.best.t, t, u, v)) {
-            const int32_t id = (kTwoLevel ? s.id_base : 0) + int32_t(__float_as_uint(c.y));
-            if (kAnyHit) {
-                s.best = TraceHit{t, u, v, id};
-                return true;
-            }
-            if (t < s.best.t || s.best.id < 0 || id < s.best.id) s.best = TraceHit{t, u, v, id};
-        }
-        // closest hit (mode 2): after the last pending triangle go on to the next node in the same
-        // step; any hit keeps one triangle per step (measured faster for shadow rays)
-        if (kAnyHit || LMGPU_TRAV_SPLIT != 2) return s.tri_mask == 0u && s.node == 0xffffffffu;
+        if (trav_test_tri<kAnyHit, kCount, false>(bvh, s)) return true;
+        // closest hit: after the last pending triangle go on to the next node in the same step; any
+        // hit keeps one triangle per step (measured faster for shadow rays)
+        if (kAnyHit) return s.tri_mask == 0u && s.node == kNoNode;
         if (s.tri_mask != 0u) return false;
     }
-    if (s.node == 0xffffffffu) return true;
+    if (s.node == kNoNode) return true;
     if (s.node >= bvh.num_nodes || s.nvis >= bvh.max_visits) { *err = 2; return true; }
     const uint4* np = bvh.nodes + size_t(s.node) * 5;
-    const uint4 w0 = __ldg(np), w1 = __ldg(np + 1);
+    const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
     s.nvis++;
-    if (kTwoLevel && (w0.w & 0xffu) == 0xffu) {
-        const float4* ip = bvh.inst + size_t(w1.x) * 4;
-        const float4 r0 = __ldg(ip), r1 = __ldg(ip + 1), r2 = __ldg(ip + 2);
-        const uint4 m = __ldg(reinterpret_cast<const uint4*>(ip + 3));
-        s.wo = s.o;
-        s.wd = s.d;
-        const f3 lo = {r0.x * s.o.x + r0.y * s.o.y + r0.z * s.o.z + r0.w, r1.x * s.o.x + r1.y * s.o.y + r1.z * s.o.z + r1.w,
-                       r2.x * s.o.x + r2.y * s.o.y + r2.z * s.o.z + r2.w};
-        const f3 ld = {r0.x * s.d.x + r0.y * s.d.y + r0.z * s.d.z, r1.x * s.d.x + r1.y * s.d.y + r1.z * s.d.z,
-                       r2.x * s.d.x + r2.y * s.d.y + r2.z * s.d.z};
-        trav_set_ray(s, lo, ld);
-        s.inst_sp = s.sp;
-        s.id_base = int32_t(m.y);
-        s.node = m.x;
-        return false;
-    }
-    const uint4 w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
-    const uint32_t oct = s.oct;
-    const float sx = __uint_as_float((w0.w & 0xffu) << 23);
-    const float sy = __uint_as_float(((w0.w >> 8) & 0xffu) << 23);
-    const float sz = __uint_as_float(((w0.w >> 16) & 0xffu) << 23);
-    const uint32_t imask = w0.w >> 24;
-    const float ax = sx * s.inv.x, ay = sy * s.inv.y, az = sz * s.inv.z;
-    const float bx = (__uint_as_float(w0.x) - s.o.x) * s.inv.x;
-    const float by = (__uint_as_float(w0.y) - s.o.y) * s.inv.y;
-    const float bz = (__uint_as_float(w0.z) - s.o.z) * s.inv.z;
-    const float ax8 = ax * 0.00390625f, ay8 = ay * 0.00390625f, az8 = az * 0.00390625f;
-    const float bx8 = fmaf(-32768.0f, ax, bx), by8 = fmaf(-32768.0f, ay, by), bz8 = fmaf(-32768.0f, az, bz);
-    const uint32_t lx0 = w2.x, lx1 = w2.y, ly0 = w2.z, ly1 = w2.w, lz0 = w3.x, lz1 = w3.y;
-    const uint32_t hx0 = w3.z, hx1 = w3.w, hy0 = w4.x, hy1 = w4.y, hz0 = w4.z, hz1 = w4.w;
-    const uint32_t nx0 = (oct & 1u) ? hx0 : lx0, nx1 = (oct & 1u) ? hx1 : lx1;
-    const uint32_t fx0 = (oct & 1u) ? lx0 : hx0, fx1 = (oct & 1u) ? lx1 : hx1;
-    const uint32_t ny0 = (oct & 2u) ? hy0 : ly0, ny1 = (oct & 2u) ? hy1 : ly1;
-    const uint32_t fy0 = (oct & 2u) ? ly0 : hy0, fy1 = (oct & 2u) ? ly1 : hy1;
-    const uint32_t nz0 = (oct & 4u) ? hz0 : lz0, nz1 = (oct & 4u) ? hz1 : lz1;
-    const uint32_t fz0 = (oct & 4u) ? lz0 : hz0, fz1 = (oct & 4u) ? lz1 : hz1;
-    uint32_t hitmask = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const uint32_t sel = 0x5404u | (uint32_t(k & 3) << 4);
-        const float qnx = __uint_as_float(__byte_perm(k < 4 ? nx0 : nx1, 0x4B00u, sel));
-        const float qfx = __uint_as_float(__byte_perm(k < 4 ? fx0 : fx1, 0x4B00u, sel));
-        const float qny = __uint_as_float(__byte_perm(k < 4 ? ny0 : ny1, 0x4B00u, sel));
-        const float qfy = __uint_as_float(__byte_perm(k < 4 ? fy0 : fy1, 0x4B00u, sel));
-        const float qnz = __uint_as_float(__byte_perm(k < 4 ? nz0 : nz1, 0x4B00u, sel));
-        const float qfz = __uint_as_float(__byte_perm(k < 4 ? fz0 : fz1, 0x4B00u, sel));
-        const float tn = fmax3(fmaf(qnx, ax8, bx8), fmaf(qny, ay8, by8), fmaxf(fmaf(qnz, az8, bz8), s.tmin));
-        const float tf0 = fmin3(fmaf(qfx, ax8, bx8), fmaf(qfy, ay8, by8), fminf(fmaf(qfz, az8, bz8), s.best.t));
-        if (tn <= tf0 * 1.0000038f) hitmask |= 1u << k;
-    }
-    // the entered leaf children's triangles, in trav_step's order (children ascending, then the
-    // triangles of each): one mask bit per triangle slot after the node's first triangle
-    uint32_t leaves = hitmask & ~imask, tmask = 0u;
-    while (leaves) {
-        const int k = __ffs(leaves) - 1;
-        leaves &= leaves - 1;
-        const uint32_t meta = byte_of(k < 4 ? w1.z : w1.w, k & 3);
-        const uint32_t cnt = meta >> 5, off = meta & 31u;
-        tmask |= ((1u << cnt) - 1u) << off;
-    }
+    const uint32_t hit = node_children(w0, w2, w3, w4, s), imask = w0.w >> 24;
     s.tri_base = w1.y;
-    s.tri_mask = tmask;
+    s.tri_mask = leaf_triangles(w1, hit & ~imask);
     // next node (visited after these triangles)
-    uint32_t inner = oct_permute(hitmask & imask, oct);
-    uint32_t g_base = w1.x, g_imask = imask;
-    if (inner == 0u) {
-        if (kTwoLevel && s.sp == s.inst_sp) {
-            // the instance is done once its last node's triangles are: test them in this frame
-            // first (a node sentinel would lose the frame switch), so finish them here
-            while (s.tri_mask) {
-                const int j = __ffs(s.tri_mask) - 1;
-                s.tri_mask &= s.tri_mask - 1u;
-                const float4* tp = bvh.tris + size_t(s.tri_base + uint32_t(j)) * 3;
-                const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
-                if (kCount) s.ntri++;
-                float t, u, v;
-                if (tri_test(s.o, s.d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), s.tmin, s.best.t, t, u, v)) {
-                    const int32_t id = s.id_base + int32_t(__float_as_uint(c.y));
-                    if (kAnyHit) {
-                        s.best = TraceHit{t, u, v, id};
-                        return true;
-                    }
-                    if (t < s.best.t || s.best.id < 0 || id < s.best.id) s.best = TraceHit{t, u, v, id};
-                }
-            }
-            trav_set_ray(s, s.wo, s.wd);
-            s.inst_sp = -1;
-            s.id_base = 0;
-        }
-        if (s.sp == 0) {
-            s.node = 0xffffffffu;  // no node left: done after the pending triangles
-            return s.tri_mask == 0u;
-        }
-        s.sp--;
-        g_base = stk_base[s.sp * stride];
-        const uint32_t bits = stk_bits[s.sp * stride];
-        g_imask = bits >> 8;
-        inner = bits & 0xffu;
-    }
-    const int k = __ffs(inner) - 1;
-    inner &= inner - 1;
-    const uint32_t slot = uint32_t(k) ^ s.oct;
-    s.node = g_base + __popc(g_imask & ((1u << slot) - 1u));
-    if (inner != 0u) {
-        if (s.sp >= bvh.depth) { *err = 1; return true; }
-        stk_base[s.sp * stride] = g_base;
-        stk_bits[s.sp * stride] = (g_imask << 8) | inner;
-        s.sp++;
-    }
-    return false;
+    if (!trav_next<false>(bvh, s, w1.x, imask, hit & imask, stk, stride)) { *err = 1; return true; }
+    return s.node == kNoNode && s.tri_mask == 0u;
 }
-#endif
 
 // One ray to the end. Adds the node visits and triangle tests to *nodes_visited / *tris_tested
 // when kCount.
 template <bool kAnyHit, bool kCount, bool kTwoLevel = false>
-__device__ inline TraceHit trace_bvh8(const Bvh8& bvh, f3 o, f3 d, float tmin, float tmax, uint32_t* stk_base,
-                                      uint32_t* stk_bits, int stride, uint32_t* nodes_visited, uint32_t* tris_tested,
-                                      int* err) {
+__device__ inline TraceHit trace_bvh8(const Bvh8& bvh, f3 o, f3 d, float tmin, float tmax, uint2* stk, int stride,
+                                      uint32_t* nodes_visited, uint32_t* tris_tested, int* err) {
     Trav s;
     trav_init(s, o, d, tmin, tmax);
-    while (!trav_step<kAnyHit, kCount, kTwoLevel>(bvh, s, stk_base, stk_bits, stride, err)) {
+    while (!trav_step<kAnyHit, kCount, kTwoLevel>(bvh, s, stk, stride, err)) {
     }
     if (kCount) { *nodes_visited += s.nvis; *tris_tested += s.ntri; }
     return s.best;
@@ -514,52 +437,207 @@ struct Fetch {
     int refill;
 };
 
+// Cooperative traversal: eight lanes per ray, four rays per warp, for launches and queue ends that
+// leave fewer rays than lanes. A lane tests one child box and one triangle, so a visit takes about
+// a third of the instructions of a lane that tests all of them, and a node's triangles are tested
+// together; what remains is the chain of dependent loads. The box and triangle tests are the
+// one-lane steps' and the smallest (t, index) wins as there, so the results are the same. The
+// longest rays take 100-200 steps of about 0.6 us, so a launch's last rays cost 100 us and more
+// whatever its size: 16k rays into a soup of 60k triangles 114 -> 89 us, 200k 195 -> 179 us, the
+// light-traced frame (18 trace launches) 3.68 -> 3.31 ms with the smaller blocks of its kernels.
+constexpr int kCoopLanes = 8, kCoopRays = 32 / kCoopLanes;
+
+// Tests the triangles s.tri_mask of each group's ray (same in the group's lanes); any hit: true in
+// the lanes of a group whose ray hits one. Called by full warps; groups without a ray: mask 0.
+template <bool kAnyHit, bool kTwoLevel>
+__device__ __forceinline__ bool coop_tris(const Bvh8& bvh, Trav& s) {
+    const unsigned sub = threadIdx.x & (kCoopLanes - 1);
+    bool found = false;
+    // a node has at most 24 triangles (8 children of at most 3)
+#pragma unroll 1
+    for (int r = 0; r < 32 && __ballot_sync(0xffffffffu, s.tri_mask != 0u); r += kCoopLanes) {
+        float t = INFINITY, u = 0.f, v = 0.f;
+        int32_t id = INT32_MAX;
+        if ((s.tri_mask >> sub) & 1u) {
+            const float4* tp = bvh.tris + size_t(s.tri_base + uint32_t(r) + sub) * 3;
+            const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+            float tt, tu, tv;
+            if (tri_test(s.o, s.d, mk(a.x, a.y, a.z), mk(a.w, b.x, b.y), mk(b.z, b.w, c.x), s.tmin, s.best.t, tt, tu, tv)) {
+                t = tt;
+                u = tu;
+                v = tv;
+                id = (kTwoLevel ? s.id_base : 0) + int32_t(__float_as_uint(c.y));
+            }
+        }
+        s.tri_mask >>= kCoopLanes;
+        if (__ballot_sync(0xffffffffu, id != INT32_MAX) == 0u) continue;
+#pragma unroll
+        for (int o = 1; o < kCoopLanes; o <<= 1) {
+            const float ot = __shfl_xor_sync(0xffffffffu, t, o), ou = __shfl_xor_sync(0xffffffffu, u, o);
+            const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+            const int32_t oi = __shfl_xor_sync(0xffffffffu, id, o);
+            if (ot < t || (!(t < ot) && oi < id)) {
+                t = ot;
+                u = ou;
+                v = ov;
+                id = oi;
+            }
+        }
+        if (id != INT32_MAX && (kAnyHit || t < s.best.t || s.best.id < 0 || id < s.best.id)) {
+            s.best = TraceHit{t, u, v, id};
+            if (kAnyHit) {
+                found = true;
+                s.tri_mask = 0u;
+            }
+        }
+    }
+    return found;
+}
+
+// Runs the groups' rays to their ends: `live` groups hold entry k in state s (the same in all lanes
+// of the group), `stk` is the stack column of the ray. Called by full warps.
+template <bool kAnyHit, bool kTwoLevel, typename End>
+__device__ __forceinline__ void coop_loop(const Bvh8& bvh, Trav& s, bool live, int k, uint2* stk, int stride, int* lerr, End end) {
+    const unsigned sub = threadIdx.x & (kCoopLanes - 1);
+    if (!live) s.tri_mask = 0u;
+    bool done = coop_tris<kAnyHit, kTwoLevel>(bvh, s);  // triangles pending from one-lane steps
+    if (live && s.node == kNoNode) done = true;
+    while (true) {
+        if (live && done) {
+            if (sub == 0u) end(k, s);
+            live = false;
+        }
+        __syncwarp();  // stack entries written by one lane are read by its group
+        if (__ballot_sync(0xffffffffu, live) == 0u) return;
+        done = false;
+        uint4 w0 = make_uint4(0u, 0u, 0u, 0u), w1 = w0;
+        bool test = false, enter = false;
+        if (live) {
+            if (s.node >= bvh.num_nodes || s.nvis >= bvh.max_visits) {
+                *lerr = 2;
+                done = true;
+            } else {
+                const uint4* np = bvh.nodes + size_t(s.node) * 5;
+                w0 = __ldg(np);
+                w1 = __ldg(np + 1);
+                s.nvis++;
+                if (kTwoLevel && (w0.w & 0xffu) == 0xffu) {
+                    trav_enter_instance(bvh, s, w1);
+                } else {
+                    test = true;
+                    // this lane's child: its near and far plane bytes (qlo x y z, then qhi x y z)
+                    const unsigned char* q = reinterpret_cast<const unsigned char*>(np + 2) + sub;
+                    const int ox = (s.oct & 1u) ? 24 : 0, oy = (s.oct & 2u) ? 24 : 0, oz = (s.oct & 4u) ? 24 : 0;
+                    auto plane = [&](int at, float a, float b) {
+                        return fmaf(__uint_as_float(0x4B000000u | (uint32_t(__ldg(q + at)) << 8)), a, b);
+                    };
+                    const Slabs S = node_slabs(w0, s);
+                    const float n = fmax3(plane(ox, S.ax, S.bx), plane(8 + oy, S.ay, S.by), fmaxf(plane(16 + oz, S.az, S.bz), s.tmin));
+                    const float f = fmin3(plane(24 - ox, S.ax, S.bx), plane(32 - oy, S.ay, S.by),
+                                          fminf(plane(40 - oz, S.az, S.bz), s.best.t));
+                    enter = !signbit(fmaf(f, kWiden, -n));
+                }
+            }
+        }
+        const uint32_t hit = (__ballot_sync(0xffffffffu, enter) >> (threadIdx.x & (32 - kCoopLanes))) & 0xffu;
+        const uint32_t imask = w0.w >> 24;
+        uint32_t tm = ((hit & ~imask) >> sub) & 1u ? leaf_bits(__byte_perm(w1.z, w1.w, sub)) : 0u;
+        tm |= __shfl_xor_sync(0xffffffffu, tm, 1);
+        tm |= __shfl_xor_sync(0xffffffffu, tm, 2);
+        tm |= __shfl_xor_sync(0xffffffffu, tm, 4);
+        s.tri_base = w1.y;
+        s.tri_mask = tm;
+        if (coop_tris<kAnyHit, kTwoLevel>(bvh, s)) done = true;
+        if (test && !done) {
+            // every lane follows the same path; one of them writes the stack
+            if (!trav_next<kTwoLevel>(bvh, s, w1.x, imask, hit & imask, stk, stride, sub == 0u)) {
+                *lerr = 1;
+                done = true;
+            }
+            if (s.node == kNoNode) done = true;
+        }
+    }
+}
+
 // Persistent traversal with dynamic ray fetch (Aila & Laine, HPG 2009): every lane of a warp
 // holds one ray in flight; once fewer than f.refill lanes still trace, the idle lanes take the
 // next entries of the queue (one atomic per warp), so a warp no longer waits for its slowest
-// ray. begin(k, s, B) loads entry k into the traversal state (and B, the BVH it traverses);
-// end(k, s) consumes the finished traversal. Called by every thread of full warps.
-template <bool kAnyHit, bool kCount, bool kTwoLevel, typename Begin, typename End>
-__device__ __forceinline__ void fetch_loop(int n, const Fetch& f, const Bvh8& bvh0, uint32_t* sb, uint32_t* sbits,
-                                           int stride, int* lerr, Begin begin, End end) {
+// ray. begin(k, s) loads entry k into the traversal state; tree(k) is the BVH it traverses;
+// end(k, s) consumes the finished traversal. Called by every thread of full warps; `warps`: the
+// warps that share the queue.
+template <bool kAnyHit, bool kCount, bool kTwoLevel, typename Begin, typename Tree, typename End>
+__device__ __forceinline__ void fetch_loop(int n, int warps, const Fetch& f, uint2* stk, int stride, int* lerr, Begin begin,
+                                           Tree tree, End end) {
     const int lane = int(threadIdx.x & 31u);
     const unsigned below = (1u << lane) - 1u;
+    // fewer rays than lanes: spread them over the warps, at least what a cooperative warp takes
+    const int lanes = n >= 32 * warps ? 32 : max(kCoopRays, (n + warps - 1) / warps);
     Trav s;
-    Bvh8 B = bvh0;
+    Bvh8 B{};
     int k = 0;
     bool active = false, exhausted = false;
     while (true) {
         if (!exhausted) {
-            const unsigned idle = __ballot_sync(0xffffffffu, !active);
+            const unsigned idle = __ballot_sync(0xffffffffu, !active && lane < lanes);
             if (idle) {
                 const int leader = __ffs(idle) - 1;
                 int base = 0;
                 if (lane == leader) base = atomicAdd(f.self, __popc(idle));
                 base = __shfl_sync(0xffffffffu, base, leader);
                 if (base + __popc(idle) >= n) exhausted = true;  // warp-uniform
-                if (!active) {
+                if ((idle >> lane) & 1u) {
                     k = base + __popc(idle & below);
                     if (k < n) {
-                        begin(k, s, B);
+                        begin(k, s);
+                        B = tree(k);
                         active = true;
                     }
                 }
             }
         }
-        if (__ballot_sync(0xffffffffu, active) == 0u) break;
-        const int keep = exhausted ? 1 : f.refill;
-        do {
-#if LMGPU_TRAV_SPLIT
+        unsigned act = __ballot_sync(0xffffffffu, active);
+        if (act == 0u) {
+            if (exhausted) return;
+            continue;
+        }
+        const int keep = exhausted ? (kCount ? 1 : kCoopRays + 1) : min(f.refill, lanes);
+        while (__popc(act) >= keep) {
             // two-level trees keep whole-node steps (measured faster on the instanced frame)
-            if (active && (kTwoLevel ? trav_step<kAnyHit, kCount, kTwoLevel>(B, s, sb, sbits, stride, lerr)
-                                     : trav_step_split<kAnyHit, kCount, kTwoLevel>(B, s, sb, sbits, stride, lerr))) {
-#else
-            if (active && trav_step<kAnyHit, kCount, kTwoLevel>(B, s, sb, sbits, stride, lerr)) {
-#endif
+            bool done = false;
+            if (active) {
+                if constexpr (kTwoLevel) done = trav_step<kAnyHit, kCount, true>(B, s, stk, stride, lerr);
+                else done = trav_step_split<kAnyHit, kCount>(B, s, stk, stride, lerr);
+            }
+            if (done) {
                 end(k, s);
                 active = false;
             }
-        } while (__popc(__ballot_sync(0xffffffffu, active)) >= keep);
+            act = __ballot_sync(0xffffffffu, active);
+        }
+        if (!kCount && exhausted && act != 0u) {
+            // hand the last rays to groups of eight lanes
+            unsigned m = act;
+            for (int g = lane / kCoopLanes; g > 0; g--) m &= m - 1u;
+            const bool live = m != 0u;
+            const int src = live ? __ffs(m) - 1 : lane;
+            auto from = [&](auto& x) { x = __shfl_sync(0xffffffffu, x, src); };
+            from(s.o.x); from(s.o.y); from(s.o.z);
+            from(s.d.x); from(s.d.y); from(s.d.z);
+            from(s.inv.x); from(s.inv.y); from(s.inv.z);
+            from(s.tmin); from(s.oct); from(s.sp); from(s.node); from(s.nvis);
+            from(s.best.t); from(s.best.u); from(s.best.v); from(s.best.id);
+            from(s.tri_base); from(s.tri_mask);
+            if (kTwoLevel) {
+                from(s.wo.x); from(s.wo.y); from(s.wo.z);
+                from(s.wd.x); from(s.wd.y); from(s.wd.z);
+                from(s.inst_sp); from(s.id_base);
+            }
+            from(k);
+            if (live) B = tree(k);
+            __syncwarp();
+            coop_loop<kAnyHit, kTwoLevel>(B, s, live, k, stk + (src - lane), stride, lerr, end);
+            return;
+        }
     }
 }
 

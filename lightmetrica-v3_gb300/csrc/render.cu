@@ -721,15 +721,13 @@ struct JobDev {
 };
 
 constexpr int kBlock = 256;
+// Trace kernels: 128-thread blocks (a block gives its registers back once its slowest ray is done),
+// seven per SM for closest hits (72 registers; eight at 64 registers spill: 2 % slower frames) and
+// eight for any hit (64 registers; nine at 56 spill: 1 %). At 256 threads and 4 / 5 blocks: 4 % slower.
+constexpr int kTrace = 128, kExtendBlocks = 7, kShadowBlocks = 8;
 // Shadow-queue pixel word: bit 31 marks an odd pass of a split-pass film (pixels stay below 2^31).
 constexpr uint32_t kOddPass = 0x80000000u;
 constexpr int64_t kRenderQueue = int64_t(1) << 25;  // paths in flight of lmgpu_render_pt by default (2^24: 1.2 % slower; 2^26: no faster)
-#ifndef LMGPU_TRACE_MINBLOCKS
-#define LMGPU_TRACE_MINBLOCKS 4  // resident 256-thread blocks per SM of the closest-hit kernel (3 and 5 measured slower)
-#endif
-#ifndef LMGPU_SHADOW_MINBLOCKS
-#define LMGPU_SHADOW_MINBLOCKS 5  // the any-hit kernel (shadow rays): 5 measured faster than 4 (24.6 -> 23.4 ms per frame)
-#endif
 
 #ifndef LMGPU_RNG_LOOP_UNROLL
 #define LMGPU_RNG_LOOP_UNROLL 4
@@ -915,29 +913,28 @@ __device__ inline void record_worst(unsigned long long* maxv, float* worst, uint
 // traverses its own job's BVH; bvh.depth is then the largest depth of the table (stack size).
 // f.refill > 0: persistent with dynamic fetch; 0: one ray per thread, grid-stride.
 template <bool kCount, bool kBatched = false, bool kTwoLevel = false>
-__global__ void __launch_bounds__(kBlock, LMGPU_TRACE_MINBLOCKS) k_pt_extend(Bvh8 bvh, const float4* __restrict__ qo, const float4* __restrict__ qd,
+__global__ void __launch_bounds__(kTrace, kExtendBlocks) k_pt_extend(Bvh8 bvh, const float4* __restrict__ qo, const float4* __restrict__ qd,
                                                       const int* __restrict__ qcount, float4* __restrict__ hits,
                                                       unsigned long long* rays, int* err, unsigned long long* sums,
                                                       int count_mask, float* worst, Fetch f, const JobDev* __restrict__ jobs = nullptr,
                                                       const uint32_t* __restrict__ qjob = nullptr) {
-    extern __shared__ uint32_t smem[];
+    extern __shared__ uint2 smem[];
     const int n = *qcount;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(rays, (unsigned long long)n);
         if (f.other) *f.other = 0;
     }
-    uint32_t* sb = smem + threadIdx.x;
-    uint32_t* sbits = smem + blockDim.x * bvh.depth + threadIdx.x;
+    uint2* stk = smem + threadIdx.x;
     int lerr = 0;
     uint32_t cn = 0, ct = 0, cc = 0;
     if (f.refill > 0) {
         fetch_loop<false, kCount, kTwoLevel>(
-            n, f, bvh, sb, sbits, int(blockDim.x), &lerr,
-            [&](int k, Trav& s, Bvh8& B) {
+            n, int(gridDim.x * (blockDim.x / 32)), f, stk, int(blockDim.x), &lerr,
+            [&](int k, Trav& s) {
                 const float4 o = qo[k], d = qd[k];
-                if (kBatched) B = jobs[qjob[k]].S.bvh;
                 trav_init(s, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, kInf);
             },
+            [&](int k) -> Bvh8 { return kBatched ? jobs[qjob[k]].S.bvh : bvh; },
             [&](int k, const Trav& s) {
                 hits[k] = make_float4(s.best.t, s.best.u, s.best.v, __int_as_float(s.best.id));
                 if (kCount && (k & count_mask) == 0) {
@@ -955,12 +952,12 @@ __global__ void __launch_bounds__(kBlock, LMGPU_TRACE_MINBLOCKS) k_pt_extend(Bvh
             TraceHit h;
             if (kCount && (k & count_mask) == 0) {
                 const uint32_t before = cn;
-                h = trace_bvh8<false, true, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, kInf, sb, sbits, blockDim.x, &cn,
+                h = trace_bvh8<false, true, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, kInf, stk, blockDim.x, &cn,
                                             &ct, &lerr);
                 cc++;
                 record_worst(sums + 6, worst, cn - before, o, d, kEps, kInf);
             } else {
-                h = trace_bvh8<false, false, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, kInf, sb, sbits, blockDim.x,
+                h = trace_bvh8<false, false, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, kInf, stk, blockDim.x,
                                              nullptr, nullptr, &lerr);
             }
             hits[k] = make_float4(h.t, h.u, h.v, __int_as_float(h.id));
@@ -977,11 +974,11 @@ __global__ void __launch_bounds__(kBlock, LMGPU_TRACE_MINBLOCKS) k_pt_extend(Bvh
 // Shadow rays: any hit over [Eps, tmax]; unoccluded contributions go to the film. kCount,
 // kBatched and f as in k_pt_extend; counts into sums[3..5].
 template <bool kCount, bool kBatched = false, bool kTwoLevel = false>
-__global__ void __launch_bounds__(kBlock, LMGPU_SHADOW_MINBLOCKS) k_pt_shadow(Bvh8 bvh, ShadowQ sq, const int* __restrict__ scount, float* film,
+__global__ void __launch_bounds__(kTrace, kShadowBlocks) k_pt_shadow(Bvh8 bvh, ShadowQ sq, const int* __restrict__ scount, float* film,
                                                       unsigned long long* rays, int* err, unsigned long long* sums,
                                                       int count_mask, float* worst, Fetch f, const JobDev* __restrict__ jobs = nullptr,
                                                       float* film_odd = nullptr) {
-    extern __shared__ uint32_t smem[];
+    extern __shared__ uint2 smem[];
     const int n = *scount;
     // the accumulator of an unoccluded contribution: the pixel word's bit 31 marks an odd pass
     auto target = [&](uint32_t job, uint32_t pw) -> float* {
@@ -992,18 +989,17 @@ __global__ void __launch_bounds__(kBlock, LMGPU_SHADOW_MINBLOCKS) k_pt_shadow(Bv
         atomicAdd(rays, (unsigned long long)n);
         if (f.other) *f.other = 0;
     }
-    uint32_t* sb = smem + threadIdx.x;
-    uint32_t* sbits = smem + blockDim.x * bvh.depth + threadIdx.x;
+    uint2* stk = smem + threadIdx.x;
     int lerr = 0;
     uint32_t cn = 0, ct = 0, cc = 0;
     if (f.refill > 0) {
         fetch_loop<true, kCount, kTwoLevel>(
-            n, f, bvh, sb, sbits, int(blockDim.x), &lerr,
-            [&](int k, Trav& s, Bvh8& B) {
+            n, int(gridDim.x * (blockDim.x / 32)), f, stk, int(blockDim.x), &lerr,
+            [&](int k, Trav& s) {
                 const float4 o = sq.o[k], d = sq.d[k];
-                if (kBatched) B = jobs[sq.job[k]].S.bvh;
                 trav_init(s, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, o.w);
             },
+            [&](int k) -> Bvh8 { return kBatched ? jobs[sq.job[k]].S.bvh : bvh; },
             [&](int k, const Trav& s) {
                 if (s.best.id < 0) {
                     const float4 c = sq.c[k];
@@ -1026,12 +1022,12 @@ __global__ void __launch_bounds__(kBlock, LMGPU_SHADOW_MINBLOCKS) k_pt_shadow(Bv
             TraceHit h;
             if (kCount && (k & count_mask) == 0) {
                 const uint32_t before = cn;
-                h = trace_bvh8<true, true, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, o.w, sb, sbits, blockDim.x, &cn,
+                h = trace_bvh8<true, true, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, o.w, stk, blockDim.x, &cn,
                                            &ct, &lerr);
                 cc++;
                 record_worst(sums + 7, worst + 8, cn - before, o, d, kEps, o.w);
             } else {
-                h = trace_bvh8<true, false, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, o.w, sb, sbits, blockDim.x,
+                h = trace_bvh8<true, false, kTwoLevel>(B, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, o.w, stk, blockDim.x,
                                             nullptr, nullptr, &lerr);
             }
             if (h.id < 0) {
@@ -1938,9 +1934,8 @@ __global__ void k_scale(const float* __restrict__ in, float* __restrict__ out, i
 // renderer::raycast, one thread per pixel (renderer_raycast.cpp:70-98)
 template <bool kTwoLevel>
 __global__ void __launch_bounds__(kBlock) k_raycast(DevScene S, int w, int h, lmgpu_raycast_params prm, float* film, int* err) {
-    extern __shared__ uint32_t smem[];
-    uint32_t* sb = smem + threadIdx.x;
-    uint32_t* sbits = smem + blockDim.x * S.bvh.depth + threadIdx.x;
+    extern __shared__ uint2 smem[];
+    uint2* stk = smem + threadIdx.x;
     int lerr = 0;
     const int64_t n = int64_t(w) * h;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
@@ -1948,7 +1943,7 @@ __global__ void __launch_bounds__(kBlock) k_raycast(DevScene S, int w, int h, lm
         const float rx = ieee::div(ieee::add(float(x), .5f), float(w)), ry = ieee::div(ieee::add(float(y), .5f), float(h));
         const f3 d = primary_dir(S, rx, ry);
         const TraceHit hit =
-            trace_bvh8<false, false, kTwoLevel>(S.bvh, S.cam_p, d, kEps, kInf, sb, sbits, blockDim.x, nullptr, nullptr, &lerr);
+            trace_bvh8<false, false, kTwoLevel>(S.bvh, S.cam_p, d, kEps, kInf, stk, blockDim.x, nullptr, nullptr, &lerr);
         f3 c;
         if (hit.id < 0) {
             if (S.env_light >= 0) {
@@ -2599,7 +2594,7 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
-        const size_t tsmem = size_t(2) * 4 * kBlock * size_t(bvh.depth);
+        const size_t tsmem = size_t(2) * 4 * kTrace * size_t(bvh.depth);
 
         const bool inst = prm->instrument != 0;
         const bool two = s->dev.num_inst > 0;
@@ -2608,8 +2603,8 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
         auto sh_k = inst ? (two ? k_pt_shadow<true, false, true> : k_pt_shadow<true, false, false>)
                          : (two ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>);
         const int g_gen = grid_for(k_pt_generate, kBlock, 0);
-        const int g_ext = grid_for(ext_k, kBlock, tsmem);
-        const int g_sh = grid_for(sh_k, kBlock, tsmem);
+        const int g_ext = grid_for(ext_k, kTrace, tsmem);
+        const int g_sh = grid_for(sh_k, kTrace, tsmem);
         auto shade_k = pick_shade(k_pt_shade<2>, k_pt_shade<3>, k_pt_shade<4>, tuning().shade_minblocks);
         const int g_shade = grid_for(shade_k, kBlock, 0);
         unsigned long long* sums = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 64);  // 8 counters
@@ -2650,7 +2645,7 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
             LMGPU_CUDA(cudaGetLastError());
             if (P.image) {
                 mark(K_SHADOW);
-                sh_k<<<g_sh, kBlock, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, sums, cmask, worst, f_sh, nullptr,
+                sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, sums, cmask, worst, f_sh, nullptr,
                                                   nullptr);
                 mark(-1);
                 n_sh++;
@@ -2658,7 +2653,7 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
             }
             for (int it = 1; it < P.max_verts; it++) {
                 mark(K_EXT);
-                ext_k<<<g_ext, kBlock, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, sums,
+                ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, sums,
                                                     cmask, worst, f_ext, nullptr, nullptr);
                 mark(-1);
                 n_ext++;
@@ -2669,7 +2664,7 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
                                                       cnt + (1 - cur), sq, cnt + 2, film);
                 mark(-1);
                 mark(K_SHADOW);
-                sh_k<<<g_sh, kBlock, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, sums, cmask, worst, f_sh, nullptr,
+                sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, sums, cmask, worst, f_sh, nullptr,
                                                   nullptr);
                 mark(-1);
                 n_sh++;
@@ -2810,7 +2805,7 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
-        const size_t tsmem = size_t(2) * 4 * kBlock * size_t(bvh.depth);
+        const size_t tsmem = size_t(2) * 4 * kTrace * size_t(bvh.depth);
         const bool two = s->dev.num_inst > 0;
         auto ext_k = two ? k_pt_extend<false, false, true> : k_pt_extend<false, false, false>;
         auto sh_k = two ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>;
@@ -2818,8 +2813,8 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
         auto shade_k = tuning().shade_minblocks >= 4 ? lt_shade_for(s->dev.feat)
                                                       : pick_shade(k_lt_shade<2>, k_lt_shade<3>, k_lt_shade<4>, tuning().shade_minblocks);
         const int g_gen = grid_for(k_lt_generate, kBlock, 0);
-        const int g_ext = grid_for(ext_k, kBlock, tsmem);
-        const int g_sh = grid_for(sh_k, kBlock, tsmem);
+        const int g_ext = grid_for(ext_k, kTrace, tsmem);
+        const int g_sh = grid_for(sh_k, kTrace, tsmem);
         const int g_shade = grid_for(shade_k, kBlock, 0);
 
         enum { K_GEN = 0, K_EXT = 1, K_SHADE = 2, K_SHADOW = 3 };
@@ -2859,7 +2854,7 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
             // the ray that leaves vertex it; its hit connects when it + 1 < max_verts
             for (int it = 1; it + 1 < P.max_verts; it++) {
                 mark(K_EXT);
-                ext_k<<<g_ext, kBlock, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
+                ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
                 mark(-1);
                 n_ext++;
@@ -2870,7 +2865,7 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
                                                       sq, cnt + 2);
                 mark(-1);
                 mark(K_SHADOW);
-                sh_k<<<g_sh, kBlock, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr,
+                sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr,
                                                   nullptr);
                 mark(-1);
                 n_sh++;
@@ -2986,15 +2981,15 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
-        const size_t tsmem = size_t(2) * 4 * kBlock * size_t(bvh.depth);
+        const size_t tsmem = size_t(2) * 4 * kTrace * size_t(bvh.depth);
         const bool two = s->dev.num_inst > 0;
         auto ext_k = two ? k_pt_extend<false, false, true> : k_pt_extend<false, false, false>;
         auto sh_k = two ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>;
         auto shade_k = tuning().shade_minblocks >= 4 ? bd_shade_for(s->dev.feat)
                                                       : pick_shade(k_bd_shade<2>, k_bd_shade<3>, k_bd_shade<4>, tuning().shade_minblocks);
         const int g_gen = grid_for(k_bd_generate, kBlock, 0);
-        const int g_ext = grid_for(ext_k, kBlock, tsmem);
-        const int g_sh = grid_for(sh_k, kBlock, tsmem);
+        const int g_ext = grid_for(ext_k, kTrace, tsmem);
+        const int g_sh = grid_for(sh_k, kTrace, tsmem);
         const int g_shade = grid_for(shade_k, kBlock, 0);
         const int g_items = grid_for(k_bd_items, kBlock, 0);
         const int g_sort = grid_for(k_bd_sort_scatter, kBlock, 0);
@@ -3041,7 +3036,7 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
                 // runs once per wave here
                 LMGPU_CUDA(cudaMemsetAsync(cnt + 4, 0, 4, st));
                 mark(K_EXT);
-                ext_k<<<g_ext, kBlock, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
+                ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
                 mark(-1);
                 n_ext++;
@@ -3068,7 +3063,7 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
             con_k<<<g_con, kBlock, 0, st>>>(s->dev, P, R, items, cnt + 6, sq, cnt + 2, scap, film, cnt + 3);
             mark(-1);
             mark(K_SHADOW);
-            sh_k<<<g_sh, kBlock, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr, nullptr);
+            sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr, nullptr);
             mark(-1);
             n_sh++;
             LMGPU_CUDA(cudaGetLastError());
@@ -3221,13 +3216,13 @@ int lmgpu_render_pt_noalloc(lmgpu_scene* s, float* d_film, int32_t w, int32_t h,
         P.w = w;
         P.h = h;
         const Bvh8 bvh = s->dev.bvh;
-        const size_t tsmem = size_t(2) * 4 * kBlock * size_t(bvh.depth);
+        const size_t tsmem = size_t(2) * 4 * kTrace * size_t(bvh.depth);
         const int g_gen = grid_for(k_pt_generate, kBlock, 0);
         const bool two = s->dev.num_inst > 0;
         auto ext_k = two ? k_pt_extend<false, false, true> : k_pt_extend<false, false, false>;
         auto sh_k = two ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>;
-        const int g_ext = grid_for(ext_k, kBlock, tsmem);
-        const int g_sh = grid_for(sh_k, kBlock, tsmem);
+        const int g_ext = grid_for(ext_k, kTrace, tsmem);
+        const int g_sh = grid_for(sh_k, kTrace, tsmem);
         auto shade_k = pick_shade(k_pt_shade<2>, k_pt_shade<3>, k_pt_shade<4>, tuning().shade_minblocks);
         const int g_shade = grid_for(shade_k, kBlock, 0);
 
@@ -3241,18 +3236,18 @@ int lmgpu_render_pt_noalloc(lmgpu_scene* s, float* d_film, int32_t w, int32_t h,
             k_pt_generate<<<std::min<int64_t>(g_gen, (n + kBlock - 1) / kBlock), kBlock, 0, st>>>(s->dev, P, start, n, q[0],
                                                                                                cnt + 0, sq, cnt + 2);
             if (P.image) {
-                sh_k<<<g_sh, kBlock, tsmem, st>>>(bvh, sq, cnt + 2, d_film, rays + 1, cnt + 3, sums, 63, nullptr, f_sh,
+                sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, d_film, rays + 1, cnt + 3, sums, 63, nullptr, f_sh,
                                                   nullptr, nullptr);
                 LMGPU_CUDA(cudaMemsetAsync(cnt + 2, 0, 4, st));
             }
             for (int it = 1; it < P.max_verts; it++) {
-                ext_k<<<g_ext, kBlock, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, hits, rays, cnt + 3, sums, 63,
+                ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, hits, rays, cnt + 3, sums, 63,
                                                     nullptr, f_ext, nullptr, nullptr);
                 LMGPU_CUDA(cudaMemsetAsync(cnt + (1 - cur), 0, 4, st));
                 LMGPU_CUDA(cudaMemsetAsync(cnt + 2, 0, 4, st));
                 shade_k<<<g_shade, kBlock, 0, st>>>(s->dev, P, q[cur], hits, cnt + cur, q[1 - cur], cnt + (1 - cur), sq,
                                                       cnt + 2, d_film);
-                sh_k<<<g_sh, kBlock, tsmem, st>>>(bvh, sq, cnt + 2, d_film, rays + 1, cnt + 3, sums, 63, nullptr, f_sh,
+                sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, d_film, rays + 1, cnt + 3, sums, 63, nullptr, f_sh,
                                                   nullptr, nullptr);
                 LMGPU_CUDA(cudaGetLastError());
                 cur = 1 - cur;
@@ -3409,7 +3404,7 @@ uint32_t table_features(const lmgpu_batch* b) {
 
 // Stream-ordered view of one chunk of iterations; captured into a graph.
 void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, bool timed) {
-    const size_t tsmem = size_t(2) * 4 * kBlock * size_t(b->max_depth);
+    const size_t tsmem = size_t(2) * 4 * kTrace * size_t(b->max_depth);
     Bvh8 bmax{};
     bmax.depth = b->max_depth;
     // one job: the plain trace kernels on its own tree and film (by value: the captured graph is
@@ -3421,8 +3416,8 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, bool timed) {
                         : (b->two_level ? k_pt_extend<false, true, true> : k_pt_extend<false, true, false>);
     auto sh_k = single ? (b->two_level ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>)
                        : (b->two_level ? k_pt_shadow<false, true, true> : k_pt_shadow<false, true, false>);
-    const int g_ext = grid_for(ext_k, kBlock, tsmem);
-    const int g_sh = grid_for(sh_k, kBlock, tsmem);
+    const int g_ext = grid_for(ext_k, kTrace, tsmem);
+    const int g_sh = grid_for(sh_k, kTrace, tsmem);
     auto shade_k = wf_shade_kernel(b, single, table_features(b));
     const int g_shade = grid_for(shade_k, kBlock, 0);
     const int g_gen = grid_for(k_wf_generate, kBlock, 0);
@@ -3455,14 +3450,14 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, bool timed) {
                                     b->alloc.as<AllocEntry>(), b->first_pass);
         k_wf_generate<<<g_gen, kBlock, 0, st>>>(jobs, b->alloc.as<AllocEntry>(), ctl64(b), q[cur], cnt + cur, sq, cnt + 2);
         mark(it, 1);
-        ext_k<<<g_ext, kBlock, tsmem, st>>>(tb, q[cur].o, q[cur].d, cnt + cur, hits, ctl_rays(b), cnt + 3, ctl_sums(b), 63,
+        ext_k<<<g_ext, kTrace, tsmem, st>>>(tb, q[cur].o, q[cur].d, cnt + cur, hits, ctl_rays(b), cnt + 3, ctl_sums(b), 63,
                                             nullptr, f_ext, single ? nullptr : jobs, single ? nullptr : q[cur].job);
         mark(it, 2);
         LMGPU_CUDA(cudaMemsetAsync(cnt + (1 - cur), 0, sizeof(int), st));
         shade_k<<<g_shade, kBlock, 0, st>>>(jobs, q[cur], hits, cnt + cur, q[1 - cur], cnt + (1 - cur), sq, cnt + 2,
                                             b->pass_done.as<unsigned int>());
         mark(it, 3);
-        sh_k<<<g_sh, kBlock, tsmem, st>>>(tb, sq, cnt + 2, sfilm, ctl_rays(b) + 1, cnt + 3, ctl_sums(b), 63, nullptr, f_sh,
+        sh_k<<<g_sh, kTrace, tsmem, st>>>(tb, sq, cnt + 2, sfilm, ctl_rays(b) + 1, cnt + 3, ctl_sums(b), 63, nullptr, f_sh,
                                           single ? nullptr : jobs, single ? J0.film_odd : nullptr);
         mark(it, 4);
         LMGPU_CUDA(cudaMemsetAsync(cnt + 2, 0, sizeof(int), st));
@@ -3500,11 +3495,11 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc) {
     cudaStream_t cs;
     LMGPU_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
     // warm-up query of grid sizes outside the capture (occupancy calls are not capturable work)
-    const size_t tsmem = size_t(2) * 4 * kBlock * size_t(b->max_depth);
-    (void)grid_for(b->two_level ? k_pt_extend<false, true, true> : k_pt_extend<false, true, false>, kBlock, tsmem);
-    (void)grid_for(b->two_level ? k_pt_shadow<false, true, true> : k_pt_shadow<false, true, false>, kBlock, tsmem);
-    (void)grid_for(b->two_level ? k_pt_extend<false, false, true> : k_pt_extend<false, false, false>, kBlock, tsmem);
-    (void)grid_for(b->two_level ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>, kBlock, tsmem);
+    const size_t tsmem = size_t(2) * 4 * kTrace * size_t(b->max_depth);
+    (void)grid_for(b->two_level ? k_pt_extend<false, true, true> : k_pt_extend<false, true, false>, kTrace, tsmem);
+    (void)grid_for(b->two_level ? k_pt_shadow<false, true, true> : k_pt_shadow<false, true, false>, kTrace, tsmem);
+    (void)grid_for(b->two_level ? k_pt_extend<false, false, true> : k_pt_extend<false, false, false>, kTrace, tsmem);
+    (void)grid_for(b->two_level ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>, kTrace, tsmem);
     (void)grid_for(wf_shade_kernel(b, single, feat), kBlock, 0);
     (void)grid_for(k_wf_generate, kBlock, 0);
     cudaGraph_t ng = nullptr;
