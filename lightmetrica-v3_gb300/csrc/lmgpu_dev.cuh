@@ -158,8 +158,8 @@ __device__ __forceinline__ float2 fma2(uint64_t a, uint64_t b, uint64_t c) {
 // one-FMA slab distances (see Slabs), so no triangle the exact test would accept is culled.
 //
 // The traversal is a resumable state (Trav) advanced one step at a time, so a persistent kernel
-// can interleave rays on a lane (dynamic ray fetch); trace_bvh8 runs one ray to the end. Either
-// way a ray's visits, tests and result are the same.
+// can interleave rays on a lane (dynamic ray fetch); trace_bvh8 runs one ray to the end. The
+// result is the same however the steps of a ray and of different rays are interleaved.
 //
 // Two-level trees (kTwoLevel): a top-level child whose node carries the instance marker
 // (exponent byte 0xFF) stands for one instance. Visiting it saves the world ray, moves the ray
@@ -180,8 +180,8 @@ struct Trav {
     f3 wo, wd;
     int inst_sp;
     int32_t id_base;
-    // split steps: the entered leaf triangles of the last node, tested one per step
-    uint32_t tri_base, tri_mask;
+    // entered leaf triangles still to be tested: of one node, and (single-level trees) of a later one
+    uint32_t tri_base, tri_mask, tri_base2, tri_mask2;
 };
 constexpr uint32_t kNoNode = 0xffffffffu;
 
@@ -209,7 +209,7 @@ __device__ inline void trav_init(Trav& s, f3 o, f3 d, float tmin, float tmax) {
     s.ntri = 0;
     s.inst_sp = -1;
     s.id_base = 0;
-    s.tri_mask = 0u;
+    s.tri_mask = s.tri_mask2 = 0u;
 }
 
 // Slab distances of one node for one ray, with one FMA per plane. Plane q of an axis lies at
@@ -387,29 +387,25 @@ __device__ __forceinline__ bool trav_step(const Bvh8& bvh, Trav& s, uint2* stk, 
     return s.node == kNoNode;
 }
 
-// trav_step with finer steps (after the triangle-postponing traversal of Ylitie et al., HPG 2017):
-// a node step records the triangles of the leaf children the ray enters as a mask; each later
-// step tests one of them; the next node is visited once the mask is empty. The order of tests is
-// trav_step's, so the result is the same; a warp's lanes now diverge between a node step and
-// one triangle test instead of waiting for the lane with the most triangles. Single-level trees.
-template <bool kAnyHit, bool kCount>
-__device__ __forceinline__ bool trav_step_split(const Bvh8& bvh, Trav& s, uint2* stk, int stride, int* err) {
-    if (s.tri_mask) {
-        if (trav_test_tri<kAnyHit, kCount, false>(bvh, s)) return true;
-        // closest hit: after the last pending triangle go on to the next node in the same step; any
-        // hit keeps one triangle per step (measured faster for shadow rays)
-        if (kAnyHit) return s.tri_mask == 0u && s.node == kNoNode;
-        if (s.tri_mask != 0u) return false;
-    }
-    if (s.node == kNoNode) return true;
+// trav_step's node part alone, for single-level trees (after the triangle postponing of Ylitie et
+// al., HPG 2017): visits s.node and only records the triangles of the entered leaf children. A ray
+// may visit further nodes while one node's triangles wait (not while two nodes' do), so a warp can
+// choose the step that most of its lanes can take; a visit before a nearer hit is known may enter
+// more nodes, the result is the same. Returns true when no node and no triangle is left.
+__device__ __forceinline__ bool trav_node(const Bvh8& bvh, Trav& s, uint2* stk, int stride, int* err) {
     if (s.node >= bvh.num_nodes || s.nvis >= bvh.max_visits) { *err = 2; return true; }
     const uint4* np = bvh.nodes + size_t(s.node) * 5;
     const uint4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3), w4 = __ldg(np + 4);
     s.nvis++;
     const uint32_t hit = node_children(w0, w2, w3, w4, s), imask = w0.w >> 24;
-    s.tri_base = w1.y;
-    s.tri_mask = leaf_triangles(w1, hit & ~imask);
-    // next node (visited after these triangles)
+    const uint32_t tmask = leaf_triangles(w1, hit & ~imask);
+    if (s.tri_mask) {
+        s.tri_base2 = w1.y;
+        s.tri_mask2 = tmask;
+    } else {
+        s.tri_base = w1.y;
+        s.tri_mask = tmask;
+    }
     if (!trav_next<false>(bvh, s, w1.x, imask, hit & imask, stk, stride)) { *err = 1; return true; }
     return s.node == kNoNode && s.tri_mask == 0u;
 }
@@ -499,8 +495,15 @@ __device__ __forceinline__ bool coop_tris(const Bvh8& bvh, Trav& s) {
 template <bool kAnyHit, bool kTwoLevel, typename End>
 __device__ __forceinline__ void coop_loop(const Bvh8& bvh, Trav& s, bool live, int k, uint2* stk, int stride, int* lerr, End end) {
     const unsigned sub = threadIdx.x & (kCoopLanes - 1);
+    // triangles pending from one-lane steps
+    const uint32_t later = live ? s.tri_mask2 : 0u;
     if (!live) s.tri_mask = 0u;
-    bool done = coop_tris<kAnyHit, kTwoLevel>(bvh, s);  // triangles pending from one-lane steps
+    bool done = coop_tris<kAnyHit, kTwoLevel>(bvh, s);
+    if (!kTwoLevel) {
+        s.tri_base = s.tri_base2;
+        s.tri_mask = done ? 0u : later;
+        done = coop_tris<kAnyHit, kTwoLevel>(bvh, s) || done;
+    }
     if (live && s.node == kNoNode) done = true;
     while (true) {
         if (live && done) {
@@ -573,6 +576,7 @@ __device__ __forceinline__ void fetch_loop(int n, int warps, const Fetch& f, uin
     // fewer rays than lanes: spread them over the warps, at least what a cooperative warp takes
     const int lanes = n >= 32 * warps ? 32 : max(kCoopRays, (n + warps - 1) / warps);
     Trav s;
+    s.tri_mask = s.tri_mask2 = 0u;
     Bvh8 B{};
     int k = 0;
     bool active = false, exhausted = false;
@@ -602,11 +606,32 @@ __device__ __forceinline__ void fetch_loop(int n, int warps, const Fetch& f, uin
         }
         const int keep = exhausted ? (kCount ? 1 : kCoopRays + 1) : min(f.refill, lanes);
         while (__popc(act) >= keep) {
-            // two-level trees keep whole-node steps (measured faster on the instanced frame)
             bool done = false;
-            if (active) {
-                if constexpr (kTwoLevel) done = trav_step<kAnyHit, kCount, true>(B, s, stk, stride, lerr);
-                else done = trav_step_split<kAnyHit, kCount>(B, s, stk, stride, lerr);
+            if constexpr (kTwoLevel || kCount) {
+                // two-level trees keep whole-node steps (a triangle must be tested before its instance
+                // is left); counted rays visit and test as trace_bvh8 does
+                if (active) done = trav_step<kAnyHit, kCount, kTwoLevel>(B, s, stk, stride, lerr);
+            } else {
+                // A triangle step when at least half as many lanes have a triangle as could visit a node.
+                // A lane's ray on a triangle idles a node step's 190 instructions and the reverse 110.
+                // 2^20 bounces in a soup of 60k triangles / 16 batched jobs: every lane with a triangle
+                // tests it before the next node 684 us / 18.3 ms; this rule at half 641 / 16.7, at one
+                // 677 / 17.4; eight lanes, whatever the number active, 678 / 17.8.
+                const unsigned tris = __ballot_sync(0xffffffffu, active && s.tri_mask != 0u);
+                const unsigned nodes = __ballot_sync(0xffffffffu, active && s.tri_mask2 == 0u && s.node != kNoNode);
+                if (2 * __popc(tris) >= __popc(nodes) || nodes == 0u) {
+                    if (active && s.tri_mask) {
+                        done = trav_test_tri<kAnyHit, kCount, false>(B, s);
+                        if (s.tri_mask == 0u) {
+                            s.tri_base = s.tri_base2;
+                            s.tri_mask = s.tri_mask2;
+                            s.tri_mask2 = 0u;
+                        }
+                        done = done || (s.tri_mask == 0u && s.node == kNoNode);
+                    }
+                } else {
+                    if (active && !done && s.tri_mask2 == 0u && s.node != kNoNode) done = trav_node(B, s, stk, stride, lerr);
+                }
             }
             if (done) {
                 end(k, s);
@@ -626,7 +651,7 @@ __device__ __forceinline__ void fetch_loop(int n, int warps, const Fetch& f, uin
             from(s.inv.x); from(s.inv.y); from(s.inv.z);
             from(s.tmin); from(s.oct); from(s.sp); from(s.node); from(s.nvis);
             from(s.best.t); from(s.best.u); from(s.best.v); from(s.best.id);
-            from(s.tri_base); from(s.tri_mask);
+            from(s.tri_base); from(s.tri_mask); from(s.tri_base2); from(s.tri_mask2);
             if (kTwoLevel) {
                 from(s.wo.x); from(s.wo.y); from(s.wo.z);
                 from(s.wd.x); from(s.wd.y); from(s.wd.z);
