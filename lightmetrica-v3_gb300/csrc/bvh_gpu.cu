@@ -22,7 +22,6 @@
 // Closest hits do not depend on the tree (the traversal's tie rule is the smaller triangle index),
 // so any of these builders gives the same hits.
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
 #include <chrono>
 #include <cmath>
@@ -178,9 +177,16 @@ __device__ void collapse_cost(const Nodes& N, int32_t id, int32_t l, int32_t r, 
     }
 }
 
+// Clusters left and the next binary node's id, kept on the device so that several passes run between
+// two reads by the host. Pass i reads state[i & 1] and leaves state[1 - (i & 1)].
+struct PlocState {
+    int32_t m, next_id;
+};
+
 // Leaves in Morton order: leaf k holds triangle vals[k]; every leaf starts as its own cluster.
 __global__ void k_leaves(const int32_t* __restrict__ vals, int64_t n, const float4* __restrict__ tlo,
-                         const float4* __restrict__ thi, Nodes N, int32_t* __restrict__ clusters) {
+                         const float4* __restrict__ thi, Nodes N, int32_t* __restrict__ clusters, PlocState* state) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *state = PlocState{int32_t(n), int32_t(n)};
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += int64_t(gridDim.x) * blockDim.x) {
         const int32_t t = vals[k];
         const float4 lo = tlo[t], hi = thi[t];
@@ -194,16 +200,63 @@ __global__ void k_leaves(const int32_t* __restrict__ vals, int64_t n, const floa
     }
 }
 
+__device__ inline float4 box_min(float4 a, float4 b) { return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), 0.f); }
+__device__ inline float4 box_max(float4 a, float4 b) { return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), 0.f); }
+
+// Area of the merged box, then the position: the order in which neighbours are preferred.
+__device__ inline unsigned long long merged_key(float4 alo, float4 ahi, float4 blo, float4 bhi, int32_t j) {
+    const float area = box_area(box_min(alo, blo), box_max(ahi, bhi));
+    return (static_cast<unsigned long long>(__float_as_uint(area)) << 32) | uint32_t(j);
+}
+
+// Exclusive prefix sum over the block's threads of (a, b) pairs packed as a << 32 | b; *total is the
+// block's sum. `shared`: one word per warp. Called by all threads of the block.
+__device__ inline unsigned long long block_scan(unsigned long long v, unsigned long long* shared, unsigned long long* total) {
+    const int lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5), warps = int(blockDim.x >> 5);
+    unsigned long long inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long u = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += u;
+    }
+    if (lane == 31) shared[warp] = inc;
+    __syncthreads();
+    unsigned long long before = 0, all = 0;
+    for (int w = 0; w < warps; w++) {
+        const unsigned long long u = shared[w];
+        before += w < warp ? u : 0ull;
+        all += u;
+    }
+    *total = all;
+    return before + inc - v;
+}
+
+// What position i does, given its nearest neighbour j and j's: a << 32 | b with a = 1 if i starts a
+// merge (a mutual pair, i the smaller position) and b = 1 if i stays a cluster (no merge, or the
+// merge's first position).
+__device__ inline unsigned long long merge_flags(int32_t i, int32_t j, int32_t nn_j) {
+    const bool mutual = j != i && nn_j == i, lead = mutual && i < j;
+    return (static_cast<unsigned long long>(lead) << 32) | ((!mutual || lead) ? 1ull : 0ull);
+}
+
 // Nearest neighbour of every cluster within kRadius places: the smallest merged surface area, ties
-// to the smaller position (a total order, so the closest pair is always mutual). Boxes of the block's
-// window are staged in shared memory.
-__global__ void __launch_bounds__(kBlock) k_nearest(const int32_t* __restrict__ clusters, int32_t m,
+// to the smaller position (a total order, so the closest pair is always mutual), and the block's
+// sums of merge_flags. Boxes and neighbours of the block's window are staged in shared memory; the
+// neighbours of kRadius places on either side are found a second time here rather than in a launch
+// of their own (a pass was five launches: neighbours, flags, a two-kernel scan and the merge).
+__global__ void __launch_bounds__(kBlock) k_nearest(const int32_t* __restrict__ clusters, const PlocState* __restrict__ state,
                                                     const float4* __restrict__ nlo, const float4* __restrict__ nhi,
-                                                    int32_t* __restrict__ nn) {
-    __shared__ float4 slo[kBlock + 2 * kRadius], shi[kBlock + 2 * kRadius];
-    const int32_t base = int32_t(blockIdx.x) * kBlock - kRadius;
-    for (int k = threadIdx.x; k < kBlock + 2 * kRadius; k += kBlock) {
-        const int32_t p = base + k;
+                                                    int32_t* __restrict__ nn, unsigned long long* __restrict__ sums) {
+    constexpr int kHalo = 2 * kRadius, kNear = kBlock + 2 * kRadius;
+    __shared__ float4 slo[kBlock + 2 * kHalo], shi[kBlock + 2 * kHalo];
+    __shared__ int32_t snn[kNear];
+    __shared__ unsigned long long warp_sum[kBlock / 32];
+    const int32_t m = state->m, first = int32_t(blockIdx.x) * kBlock;
+    if (first >= m) {
+        if (threadIdx.x == 0) sums[blockIdx.x] = 0ull;
+        return;
+    }
+    for (int k = threadIdx.x; k < kBlock + 2 * kHalo; k += kBlock) {
+        const int32_t p = first - kHalo + k;
         if (p >= 0 && p < m) {
             const int32_t c = clusters[p];
             slo[k] = nlo[c];
@@ -211,65 +264,166 @@ __global__ void __launch_bounds__(kBlock) k_nearest(const int32_t* __restrict__ 
         }
     }
     __syncthreads();
-    const int32_t i = int32_t(blockIdx.x) * kBlock + threadIdx.x;
-    if (i >= m) return;
-    const int li = threadIdx.x + kRadius;
-    const float4 alo = slo[li], ahi = shi[li];
-    unsigned long long best = ~0ull;
-    const int32_t j0 = max(0, i - kRadius), j1 = min(m - 1, i + kRadius);
-    for (int32_t j = j0; j <= j1; j++) {
-        if (j == i) continue;
-        const int lj = j - base;
-        const float4 blo = slo[lj], bhi = shi[lj];
-        const float4 ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.f);
-        const float4 uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.f);
-        const unsigned long long key = (static_cast<unsigned long long>(__float_as_uint(box_area(ulo, uhi))) << 32) |
-                                       uint32_t(j);
-        best = key < best ? key : best;
+    for (int k = threadIdx.x; k < kNear; k += kBlock) {
+        const int32_t i = first - kRadius + k;
+        if (i < 0 || i >= m) continue;
+        const float4 alo = slo[k + kRadius], ahi = shi[k + kRadius];
+        unsigned long long best = ~0ull;
+        for (int32_t j = max(0, i - kRadius); j <= min(m - 1, i + kRadius); j++) {
+            if (j == i) continue;
+            const unsigned long long key = merged_key(alo, ahi, slo[j - first + kHalo], shi[j - first + kHalo], j);
+            best = key < best ? key : best;
+        }
+        snn[k] = m > 1 ? int32_t(best & 0xffffffffu) : i;
     }
-    nn[i] = m > 1 ? int32_t(best & 0xffffffffu) : i;
+    __syncthreads();
+    const int32_t i = first + int32_t(threadIdx.x);
+    unsigned long long f = 0ull, total;
+    if (i < m) {
+        const int32_t j = snn[threadIdx.x + kRadius];
+        nn[i] = j;
+        f = merge_flags(i, j, snn[j - first + kRadius]);
+    }
+    block_scan(f, warp_sum, &total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
-// flags[i]: bit 32 = i starts a merge (mutual pair, i the smaller position); bit 0 = i stays a
-// cluster (no merge, or the merge's first position).
-__global__ void k_merge_flags(const int32_t* __restrict__ nn, int32_t m, unsigned long long* __restrict__ flags) {
-    const int32_t i = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const int32_t j = nn[i];
-    const bool mutual = j != i && nn[j] == i;
-    const bool lead = mutual && i < j;
-    flags[i] = (static_cast<unsigned long long>(lead) << 32) | ((!mutual || lead) ? 1ull : 0ull);
+// Prefix sums of the blocks' sums, in place, and the state after the pass.
+__global__ void __launch_bounds__(1024) k_scan_blocks(unsigned long long* sums, int32_t blocks, const PlocState* __restrict__ state,
+                                                      PlocState* next) {
+    __shared__ unsigned long long warp_sum[32];
+    unsigned long long run = 0;
+    for (int32_t base = 0; base < blocks; base += 1024) {
+        const int32_t k = base + int32_t(threadIdx.x);
+        unsigned long long total;
+        const unsigned long long v = k < blocks ? sums[k] : 0ull, ex = block_scan(v, warp_sum, &total);
+        if (k < blocks) sums[k] = run + ex;
+        run += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *next = PlocState{int32_t(run & 0xffffffffu), state->next_id + int32_t(run >> 32)};
 }
 
-__global__ void k_merge(const int32_t* __restrict__ cin, int32_t m, const int32_t* __restrict__ nn,
-                        const unsigned long long* __restrict__ flags, const unsigned long long* __restrict__ scan,
-                        int32_t next_id, Nodes N, int32_t* __restrict__ cout, unsigned long long* totals, int W) {
-    const int32_t i = int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const unsigned long long f = flags[i], s = scan[i];
-    if (i == m - 1) *totals = s + f;
+// The merge of clusters a and b as binary node `id` with box (lo, hi).
+__device__ inline void merge_node(const Nodes& N, int32_t id, int32_t a, int32_t b, float4 lo, float4 hi, int W) {
+    const int32_t cnt = N.count[a] + N.count[b];
+    N.lo[id] = lo;
+    N.hi[id] = hi;
+    N.left[id] = a;
+    N.right[id] = b;
+    N.count[id] = cnt;
+    collapse_cost(N, id, a, b, lo, hi, cnt, W);
+}
+__global__ void __launch_bounds__(kBlock) k_merge(const int32_t* __restrict__ cin, const PlocState* __restrict__ state,
+                                                  const int32_t* __restrict__ nn, const unsigned long long* __restrict__ before,
+                                                  Nodes N, int32_t* __restrict__ cout, int W) {
+    __shared__ unsigned long long warp_sum[kBlock / 32];
+    const int32_t i = int32_t(blockIdx.x) * kBlock + int32_t(threadIdx.x), m = state->m;
+    if (int32_t(blockIdx.x) * kBlock >= m) return;
+    const int32_t j = i < m ? nn[i] : i;
+    const unsigned long long f = i < m ? merge_flags(i, j, nn[j]) : 0ull;
+    unsigned long long total;
+    const unsigned long long s = before[blockIdx.x] + block_scan(f, warp_sum, &total);
     if (!(f & 1ull)) return;
     const int32_t slot = int32_t(s & 0xffffffffu);
     if (f >> 32) {
-        const int32_t id = next_id + int32_t(s >> 32);
-        const int32_t a = cin[i], b = cin[nn[i]];
-        const float4 alo = N.lo[a], ahi = N.hi[a], blo = N.lo[b], bhi = N.hi[b];
-        const float4 lo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.f);
-        const float4 hi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.f);
-        const int32_t cnt = N.count[a] + N.count[b];
-        N.lo[id] = lo;
-        N.hi[id] = hi;
-        N.left[id] = a;
-        N.right[id] = b;
-        N.count[id] = cnt;
-        collapse_cost(N, id, a, b, lo, hi, cnt, W);
+        const int32_t id = state->next_id + int32_t(s >> 32);
+        const int32_t a = cin[i], b = cin[j];
+        merge_node(N, id, a, b, box_min(N.lo[a], N.lo[b]), box_max(N.hi[a], N.hi[b]), W);
         cout[slot] = id;
     } else {
         cout[slot] = cin[i];
     }
 }
 
+// The root and what the host reports about it.
+struct RootInfo {
+    int32_t root;
+    float cost;
+    float lo[3], hi[3];
+};
+
+// The last kLast clusters: every remaining pass in one block, positions and boxes in shared memory,
+// the same merges and node ids as the passes above. A pass shrinks the list by about a quarter, so
+// more than half of a build's passes have fewer clusters than one block has threads; as five
+// launches and a read by the host each they took 40 us, here about 4.
+constexpr int kLast = 1024;
+__global__ void __launch_bounds__(kLast) k_last_passes(const int32_t* __restrict__ clusters, const PlocState* __restrict__ state,
+                                                       Nodes N, int W, RootInfo* out, int* err) {
+    __shared__ float4 slo[kLast], shi[kLast];
+    __shared__ int32_t sid[kLast], snn[kLast];
+    __shared__ unsigned long long warp_sum[32];
+    const int i = int(threadIdx.x);
+    int m = state->m, next_id = state->next_id;
+    if (i < m) {
+        const int32_t c = clusters[i];
+        sid[i] = c;
+        slo[i] = N.lo[c];
+        shi[i] = N.hi[c];
+    }
+    __syncthreads();
+    while (m > 1) {
+        if (i < m) {
+            unsigned long long best = ~0ull;
+            const float4 alo = slo[i], ahi = shi[i];
+            for (int j = max(0, i - kRadius); j <= min(m - 1, i + kRadius); j++) {
+                if (j == i) continue;
+                const unsigned long long key = merged_key(alo, ahi, slo[j], shi[j], j);
+                best = key < best ? key : best;
+            }
+            snn[i] = int32_t(best & 0xffffffffu);
+        }
+        __syncthreads();
+        const int j = i < m ? snn[i] : i;
+        const unsigned long long f = i < m ? merge_flags(i, j, snn[j]) : 0ull;
+        const bool keep = f & 1ull, lead = f >> 32;
+        unsigned long long total;
+        const unsigned long long ex = block_scan(f, warp_sum, &total);
+        int32_t id = 0;
+        float4 lo, hi;
+        if (keep) {
+            id = sid[i];
+            lo = slo[i];
+            hi = shi[i];
+            if (lead) {
+                const int32_t a = id, b = sid[j];
+                id = next_id + int32_t(ex >> 32);
+                lo = box_min(lo, slo[j]);
+                hi = box_max(hi, shi[j]);
+                merge_node(N, id, a, b, lo, hi, W);
+            }
+        }
+        const int merges = int(total >> 32), left = int(total & 0xffffffffu);
+        if (merges < 1 || left != m - merges) {  // the same in all threads
+            if (i == 0) atomicOr(err, kErrLayout);
+            break;
+        }
+        __syncthreads();
+        if (keep) {
+            const int slot = int(ex & 0xffffffffu);
+            sid[slot] = id;
+            slo[slot] = lo;
+            shi[slot] = hi;
+        }
+        m = left;
+        next_id += merges;
+        __syncthreads();
+    }
+    if (i == 0) {
+        const int32_t r = sid[0];
+        const float4 lo = slo[0], hi = shi[0];
+        *out = RootInfo{r, N.cost[size_t(r) * 8], {lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}};
+    }
+}
+
 // ---- emission ------------------------------------------------------------------------------
+
+// Counters of the emission, one host read for all of them.
+struct EmitState {
+    int err;
+    int32_t wide_count, tri_count;
+    int32_t level[8];  // ring: level l holds the wide nodes [level[l & 7], level[(l + 1) & 7])
+};
 
 struct Emit {
     Nodes N;
@@ -278,11 +432,9 @@ struct Emit {
     float4* tris;            // 3 float4 per triangle record
     int32_t* tri_slot;       // flattened triangle index -> record
     int32_t* q_bin;          // wide node -> its binary node
-    int32_t* wide_count;
-    int32_t* tri_count;
-    int32_t root;
+    EmitState* st;
+    const RootInfo* root;
     int32_t wide_cap;
-    int* err;
     int width;               // children per node (2..8)
 };
 
@@ -297,185 +449,267 @@ __device__ int exponent_for(double v) {
     return min(254, max(1, eb));
 }
 
-// bvh_build.cpp quantize_axis, with the margin check in double: lo, hi, p are floats and
-// q * 2^(eb-127) a multiple of the quantum, which the exponent choice keeps within 2^-45 of |p|,
-// so p + q * s is exact in double.
-__device__ bool quantize_axis(float lo, const float4* clo, const float4* chi, const bool* valid, int a, int eb,
-                              float& origin, uint8_t* qlo, uint8_t* qhi) {
-    const double s = ldexp(1.0, eb - 127);
-    const double pd = double(lo) - 2.0 * s;
-    float p = __double2float_rn(pd);
-    if (double(p) > pd) p = nextafterf(p, -INFINITY);
-    if (!(double(p) < double(lo) - s)) return false;
-    for (int k = 0; k < 8; k++) {
-        if (!valid[k]) { qlo[k] = 255; qhi[k] = 0; continue; }
-        const float bl = a == 0 ? clo[k].x : (a == 1 ? clo[k].y : clo[k].z);
-        const float bh = a == 0 ? chi[k].x : (a == 1 ? chi[k].y : chi[k].z);
-        const double l = (double(bl) - double(p)) / s;
-        const double h = (double(bh) - double(p)) / s;
-        const double ql = floor(l) - 1.0, qh = ceil(h) + 1.0;
-        if (ql < 0.0 || qh > 255.0) return false;
-        const double pl = double(p) + ql * s, ph = double(p) + qh * s;
-        if (pl + s > double(bl) || ph - s < double(bh)) return false;
-        qlo[k] = uint8_t(ql);
-        qhi[k] = uint8_t(qh);
-    }
-    origin = p;
-    return true;
-}
-
-__global__ void k_emit(Emit E, int32_t w0, int32_t w1) {
-    const int32_t w = w0 + int32_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (w >= w1) return;
+// Eight lanes per wide node, lane s for child slot s. One thread per node ran the slot assignment and
+// the quantization (both in double, as on the host, and double is slow here) for its eight children
+// in turn: 250 us per level of a 200k-triangle build however few nodes it had, 55 us now.
+constexpr int kEmitBlock = 128;
+__global__ void __launch_bounds__(kEmitBlock) k_emit(Emit E, int level) {
     const Nodes& N = E.N;
-    const int32_t bin = E.q_bin[w];
-    // children of this wide node (binary node ids) and whether each is a leaf
-    int32_t ch[8];
-    bool leaf[8];
-    int nch = 0;
-    if (N.left[bin] < 0 || (bin == E.root && N.dec[size_t(bin) * 8] == 0)) {
-        ch[0] = bin;
-        leaf[0] = true;
-        nch = 1;
-    } else {
-        // depth-first over (binary node, slots), left before right
-        int32_t sm[16];
-        int si[16];
-        int sp = 0;
-        const int k0 = N.dnode[bin];
-        sm[sp] = N.right[bin]; si[sp++] = E.width - k0;
-        sm[sp] = N.left[bin]; si[sp++] = k0;
-        while (sp > 0) {
-            const int32_t m = sm[--sp];
-            int i = si[sp];
-            while (i > 1 && N.dec[size_t(m) * 8 + i - 1] == 0) i--;
-            if (i == 1) {
-                if (nch >= 8) { atomicOr(E.err, kErrLayout); return; }
-                ch[nch] = m;
-                leaf[nch] = N.left[m] < 0 || N.dec[size_t(m) * 8] == 0;
-                nch++;
-                continue;
+    const int lane = int(threadIdx.x & 31u), s = lane & 7;
+    const unsigned gm = 0xffu << (lane & 24);
+    const int32_t w1 = E.st->level[(level + 1) & 7], root = E.root->root;
+    auto from = [&](auto v, int src) { return __shfl_sync(gm, v, src, 8); };
+    for (int32_t w = E.st->level[level & 7] + (int32_t(blockIdx.x) * kEmitBlock + int32_t(threadIdx.x)) / 8; w < w1;
+         w += int32_t(gridDim.x) * (kEmitBlock / 8)) {
+        const int32_t bin = E.q_bin[w];
+        // the node's children (binary node ids), depth-first left before right: child i goes to lane i
+        int32_t ch = -1;
+        bool leaf = false;
+        int nch = 0;
+        bool bad = false;
+        if (N.left[bin] < 0 || (bin == root && N.dec[size_t(bin) * 8] == 0)) {
+            if (s == 0) {
+                ch = bin;
+                leaf = true;
             }
-            const int k = N.dec[size_t(m) * 8 + i - 1];
-            if (sp + 2 > 16) { atomicOr(E.err, kErrLayout); return; }
-            sm[sp] = N.right[m]; si[sp++] = i - k;
-            sm[sp] = N.left[m]; si[sp++] = k;
-        }
-    }
-    // octant-ordered slots (bvh_build.cpp: greedy on dot(centroid - center, octant direction))
-    float4 nlo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), nhi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-    for (int i = 0; i < nch; i++) {
-        const float4 a = N.lo[ch[i]], b = N.hi[ch[i]];
-        nlo = make_float4(fminf(nlo.x, a.x), fminf(nlo.y, a.y), fminf(nlo.z, a.z), 0.f);
-        nhi = make_float4(fmaxf(nhi.x, b.x), fmaxf(nhi.y, b.y), fmaxf(nhi.z, b.z), 0.f);
-    }
-    const float ctr[3] = {0.5f * (nlo.x + nhi.x), 0.5f * (nlo.y + nhi.y), 0.5f * (nlo.z + nhi.z)};
-    int child_in[8];
-    bool used[8];
-    for (int s = 0; s < 8; s++) { child_in[s] = -1; used[s] = false; }
-    for (int k = 0; k < nch; k++) {
-        int bi = -1, bs = -1;
-        double bc = INFINITY;
-        for (int i = 0; i < nch; i++) {
-            if (used[i]) continue;
-            const float4 a = N.lo[ch[i]], b = N.hi[ch[i]];
-            const double dc[3] = {0.5 * (double(a.x) + b.x) - ctr[0], 0.5 * (double(a.y) + b.y) - ctr[1],
-                                  0.5 * (double(a.z) + b.z) - ctr[2]};
-            for (int s = 0; s < 8; s++) {
-                if (child_in[s] >= 0) continue;
-                double c = 0;
-                for (int ax = 0; ax < 3; ax++) c += ((s >> ax) & 1) ? -dc[ax] : dc[ax];
-                if (c < bc) { bc = c; bi = i; bs = s; }
+            nch = 1;
+        } else {
+            int32_t sm[16];
+            int si[16];
+            int sp = 0;
+            const int k0 = N.dnode[bin];
+            sm[sp] = N.right[bin]; si[sp++] = E.width - k0;
+            sm[sp] = N.left[bin]; si[sp++] = k0;
+            while (sp > 0 && !bad) {
+                const int32_t m = sm[--sp];
+                int i = si[sp];
+                while (i > 1 && N.dec[size_t(m) * 8 + i - 1] == 0) i--;
+                if (i == 1) {
+                    if (nch >= 8) { bad = true; break; }
+                    if (nch == s) {
+                        ch = m;
+                        leaf = N.left[m] < 0 || N.dec[size_t(m) * 8] == 0;
+                    }
+                    nch++;
+                    continue;
+                }
+                const int k = N.dec[size_t(m) * 8 + i - 1];
+                if (sp + 2 > 16) { bad = true; break; }
+                sm[sp] = N.right[m]; si[sp++] = i - k;
+                sm[sp] = N.left[m]; si[sp++] = k;
             }
         }
-        used[bi] = true;
-        child_in[bs] = bi;
-    }
-    // slots for internal children (contiguous wide nodes) and leaf triangles (contiguous records)
-    int nint = 0, ntri = 0;
-    for (int i = 0; i < nch; i++) {
-        if (leaf[i]) ntri += N.count[ch[i]];
-        else nint++;
-    }
-    const int32_t child_base = nint ? atomicAdd(E.wide_count, nint) : 0;
-    const int32_t tri_base = ntri ? atomicAdd(E.tri_count, ntri) : 0;
-    if (child_base + nint > E.wide_cap) { atomicOr(E.err, kErrLayout); return; }
-    uint8_t imask = 0, meta[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    float4 clo[8], chi[8];
-    bool valid[8];
-    int ki = 0, off = 0;
-    for (int s = 0; s < 8; s++) {
-        valid[s] = false;
-        const int i = child_in[s];
-        if (i < 0) continue;
-        valid[s] = true;
-        clo[s] = N.lo[ch[i]];
-        chi[s] = N.hi[ch[i]];
-        if (!leaf[i]) {
-            imask |= uint8_t(1u << s);
-            meta[s] = 0x80;
-            E.q_bin[child_base + ki] = ch[i];
-            ki++;
+        if (bad) {  // the same in all lanes of the group
+            atomicOr(&E.st->err, kErrLayout);
             continue;
         }
-        const int cnt = N.count[ch[i]];
-        if (cnt < 1 || cnt > kMaxLeaf || off > 31) { atomicOr(E.err, kErrLayout); return; }
-        meta[s] = uint8_t((cnt << 5) | off);
-        // the leaf's triangles, left to right
-        int32_t st[8];
-        int sp = 0;
-        st[sp++] = ch[i];
-        while (sp > 0) {
-            const int32_t m = st[--sp];
-            if (N.left[m] < 0) {
-                const int32_t t = N.right[m];
-                const float* p = E.P + 9 * int64_t(t);
-                const float p1x = p[0], p1y = p[1], p1z = p[2];
-                const float4 a = make_float4(p1x, p1y, p1z, __fsub_rn(p[3], p1x));
-                const float4 b = make_float4(__fsub_rn(p[4], p1y), __fsub_rn(p[5], p1z), __fsub_rn(p[6], p1x),
-                                             __fsub_rn(p[7], p1y));
-                const float4 c = make_float4(__fsub_rn(p[8], p1z), __uint_as_float(uint32_t(t)), 0.f, 0.f);
-                const int32_t rec = tri_base + off;
-                E.tris[size_t(rec) * 3] = a;
-                E.tris[size_t(rec) * 3 + 1] = b;
-                E.tris[size_t(rec) * 3 + 2] = c;
-                E.tri_slot[t] = rec;
-                off++;
-                continue;
+        // octant-ordered slots (bvh_build.cpp: greedy on dot(centroid - center, octant direction))
+        float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+        int cnt = 0;
+        if (ch >= 0) {
+            lo = N.lo[ch];
+            hi = N.hi[ch];
+            cnt = N.count[ch];
+        }
+        float4 nlo = lo, nhi = hi;
+        for (int o = 1; o < 8; o <<= 1) {
+            auto other = [&](float v) { return __shfl_xor_sync(gm, v, o); };
+            nlo = box_min(nlo, make_float4(other(nlo.x), other(nlo.y), other(nlo.z), 0.f));
+            nhi = box_max(nhi, make_float4(other(nhi.x), other(nhi.y), other(nhi.z), 0.f));
+        }
+        const float ctr[3] = {0.5f * (nlo.x + nhi.x), 0.5f * (nlo.y + nhi.y), 0.5f * (nlo.z + nhi.z)};
+        const double dc[3] = {0.5 * (double(lo.x) + hi.x) - ctr[0], 0.5 * (double(lo.y) + hi.y) - ctr[1],
+                              0.5 * (double(lo.z) + hi.z) - ctr[2]};
+        // as integers of the same order: the assignment compares them some 70 times (+ 0.0: -0 is 0)
+        unsigned long long cost[8];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            double c = (t & 1) ? -dc[0] : dc[0];
+            c += (t & 2) ? -dc[1] : dc[1];
+            c += (t & 4) ? -dc[2] : dc[2];
+            const long long bits = __double_as_longlong(c + 0.0);
+            cost[t] = static_cast<unsigned long long>(bits) ^ (bits < 0 ? ~0ull : 1ull << 63);
+        }
+        uint32_t taken = 0u;         // slots given out
+        unsigned long long map = 0;  // slot -> child, a byte each
+        bool placed = ch < 0;
+        for (int k = 0; k < nch; k++) {
+            // the smallest cost over unplaced children and free slots, ties to the smaller child, then slot
+            unsigned long long bc = ~0ull;
+            int bi = s, bs = 8;
+#pragma unroll
+            for (int t = 0; t < 8; t++)
+                if (!placed && !((taken >> t) & 1u) && cost[t] < bc) {
+                    bc = cost[t];
+                    bs = t;
+                }
+            if (bs == 8) bi = 8;  // nothing to offer
+            for (int o = 1; o < 8; o <<= 1) {
+                const unsigned long long oc = __shfl_xor_sync(gm, bc, o);
+                const int oi = __shfl_xor_sync(gm, bi, o), os = __shfl_xor_sync(gm, bs, o);
+                if (oc < bc || (oc == bc && oi < bi)) {
+                    bc = oc;
+                    bi = oi;
+                    bs = os;
+                }
             }
-            if (sp + 2 > 8) { atomicOr(E.err, kErrLayout); return; }
-            st[sp++] = N.right[m];
-            st[sp++] = N.left[m];
+            if (bi > 7) { bad = true; break; }  // no finite cost is left (the same in all lanes)
+            taken |= 1u << bs;
+            map |= static_cast<unsigned long long>(bi) << (8 * bs);
+            if (s == bi) placed = true;
+        }
+        if (bad) {
+            atomicOr(&E.st->err, kErrLayout);
+            continue;
+        }
+        // lane s takes over the child of slot s
+        const bool valid = (taken >> s) & 1u;
+        const int src = valid ? int((map >> (8 * s)) & 0xffu) : s;
+        lo = make_float4(from(lo.x, src), from(lo.y, src), from(lo.z, src), 0.f);
+        hi = make_float4(from(hi.x, src), from(hi.y, src), from(hi.z, src), 0.f);
+        ch = from(ch, src);
+        cnt = from(cnt, src);
+        leaf = from(int(leaf), src) != 0;
+        const bool is_leaf = valid && leaf;
+        const uint32_t imask = (__ballot_sync(gm, valid && !leaf) >> (lane & 24)) & 0xffu;
+        // slots for internal children (contiguous wide nodes) and leaf triangles (contiguous records)
+        const int mine = is_leaf ? cnt : 0;
+        int off = mine;
+        for (int o = 1; o < 8; o <<= 1) {
+            const int v = __shfl_up_sync(gm, off, o, 8);
+            if (s >= o) off += v;
+        }
+        const int nint = __popc(imask), ntri = from(off, 7);
+        off -= mine;
+        int32_t child_base = 0, tri_base = 0;
+        if (s == 0) {
+            child_base = nint ? atomicAdd(&E.st->wide_count, nint) : 0;
+            tri_base = ntri ? atomicAdd(&E.st->tri_count, ntri) : 0;
+        }
+        child_base = from(child_base, 0);
+        tri_base = from(tri_base, 0);
+        if (__any_sync(gm, child_base + nint > E.wide_cap || (is_leaf && (cnt < 1 || cnt > kMaxLeaf || off > 31)))) {
+            atomicOr(&E.st->err, kErrLayout);
+            continue;
+        }
+        uint32_t meta = 0u;
+        if (valid && !leaf) {
+            meta = 0x80u;
+            E.q_bin[child_base + __popc(imask & ((1u << s) - 1u))] = ch;
+        } else if (is_leaf) {
+            meta = uint32_t((cnt << 5) | off);
+            // the leaf's triangles, left to right
+            int32_t st[8];
+            int sp = 0;
+            st[sp++] = ch;
+            int32_t rec = tri_base + off;
+            while (sp > 0) {
+                const int32_t m = st[--sp];
+                if (N.left[m] < 0) {
+                    const int32_t t = N.right[m];
+                    const float* p = E.P + 9 * int64_t(t);
+                    const float p1x = p[0], p1y = p[1], p1z = p[2];
+                    E.tris[size_t(rec) * 3] = make_float4(p1x, p1y, p1z, __fsub_rn(p[3], p1x));
+                    E.tris[size_t(rec) * 3 + 1] = make_float4(__fsub_rn(p[4], p1y), __fsub_rn(p[5], p1z), __fsub_rn(p[6], p1x),
+                                                              __fsub_rn(p[7], p1y));
+                    E.tris[size_t(rec) * 3 + 2] = make_float4(__fsub_rn(p[8], p1z), __uint_as_float(uint32_t(t)), 0.f, 0.f);
+                    E.tri_slot[t] = rec;
+                    rec++;
+                    continue;
+                }
+                if (sp + 2 > 8) { bad = true; break; }
+                st[sp++] = N.right[m];
+                st[sp++] = N.left[m];
+            }
+        }
+        __syncwarp(gm);
+        // Quantization (bvh_build.cpp quantize), with the margin check in double: lo, hi and p are
+        // floats and q * 2^(eb-127) a multiple of the quantum, which the exponent choice keeps within
+        // 2^-45 of |p|, so p + q * quantum is exact in double.
+        uint32_t eb[3];
+        float origin[3];
+        uint32_t ql[3], qh[3];
+        const float nl[3] = {nlo.x, nlo.y, nlo.z}, nh[3] = {nhi.x, nhi.y, nhi.z};
+        const float bl[3] = {lo.x, lo.y, lo.z}, bh[3] = {hi.x, hi.y, hi.z};
+        bool quantized = true;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const double ext = double(nh[a]) - double(nl[a]);
+            const double mag = fmax(fabs(double(nl[a])), fabs(double(nh[a])));
+            bool ok = false;
+            for (int e = max(exponent_for(ext / 251.0), exponent_for(mag * 1.2e-7)); e <= 254 && !ok; e++) {
+                // the quantum and its inverse, both powers of two (the product is the quotient)
+                const double q = __hiloint2double((e - 127 + 1023) << 20, 0), iq = __hiloint2double((127 - e + 1023) << 20, 0);
+                const double pd = double(nl[a]) - 2.0 * q;
+                float p = __double2float_rn(pd);
+                if (double(p) > pd) p = nextafterf(p, -INFINITY);
+                bool fits = double(p) < double(nl[a]) - q;
+                uint32_t l8 = 255u, h8 = 0u;  // an empty slot's inverted box
+                if (fits && valid) {
+                    const double l = floor((double(bl[a]) - double(p)) * iq) - 1.0, h = ceil((double(bh[a]) - double(p)) * iq) + 1.0;
+                    fits = !(l < 0.0 || h > 255.0) && !(double(p) + l * q + q > double(bl[a]) || double(p) + h * q - q < double(bh[a]));
+                    if (fits) {
+                        l8 = uint32_t(l);
+                        h8 = uint32_t(h);
+                    }
+                }
+                ok = __all_sync(gm, fits);
+                if (ok) {
+                    eb[a] = uint32_t(e);
+                    origin[a] = p;
+                    ql[a] = l8;
+                    qh[a] = h8;
+                }
+            }
+            quantized = quantized && ok;
+        }
+        if (__any_sync(gm, bad)) {
+            atomicOr(&E.st->err, kErrLayout);
+            continue;
+        }
+        if (!quantized) {  // the same in all lanes of the group
+            atomicOr(&E.st->err, kErrQuantize);
+            continue;
+        }
+        // four slots' bytes per word: lanes 0-3 the first, 4-7 the second
+        auto word = [&](uint32_t v) {
+            v <<= 8 * (s & 3);
+            v |= __shfl_xor_sync(gm, v, 1);
+            return v | __shfl_xor_sync(gm, v, 2);
+        };
+        uint32_t* o = E.nodes + size_t(w) * 20;
+        const uint32_t mw = word(meta);
+        uint32_t lw[3], hw[3];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            lw[a] = word(ql[a]);
+            hw[a] = word(qh[a]);
+        }
+        if (s == 0) {
+            o[0] = fbits(origin[0]); o[1] = fbits(origin[1]); o[2] = fbits(origin[2]);
+            o[3] = eb[0] | (eb[1] << 8) | (eb[2] << 16) | (imask << 24);
+            o[4] = uint32_t(child_base);
+            o[5] = uint32_t(tri_base);
+        }
+        if ((s & 3) == 0) {
+            const int half = s >> 2;
+            o[6 + half] = mw;
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                o[8 + 2 * a + half] = lw[a];
+                o[14 + 2 * a + half] = hw[a];
+            }
         }
     }
-    // quantize (bvh_build.cpp quantize)
-    int eb[3];
-    float origin[3];
-    uint8_t qlo[3][8], qhi[3][8];
-    const float nl[3] = {nlo.x, nlo.y, nlo.z}, nh[3] = {nhi.x, nhi.y, nhi.z};
-    for (int a = 0; a < 3; a++) {
-        const double ext = double(nh[a]) - double(nl[a]);
-        const double mag = fmax(fabs(double(nl[a])), fabs(double(nh[a])));
-        int e = max(exponent_for(ext / 251.0), exponent_for(mag * 1.2e-7));
-        bool ok = false;
-        for (; e <= 254 && !ok; e++) {
-            ok = quantize_axis(nl[a], clo, chi, valid, a, e, origin[a], qlo[a], qhi[a]);
-            if (ok) eb[a] = e;
-        }
-        if (!ok) { atomicOr(E.err, kErrQuantize); return; }
-    }
-    uint32_t* o = E.nodes + size_t(w) * 20;
-    auto pack4 = [](const uint8_t* b) {
-        return uint32_t(b[0]) | (uint32_t(b[1]) << 8) | (uint32_t(b[2]) << 16) | (uint32_t(b[3]) << 24);
-    };
-    o[0] = fbits(origin[0]); o[1] = fbits(origin[1]); o[2] = fbits(origin[2]);
-    o[3] = uint32_t(eb[0]) | (uint32_t(eb[1]) << 8) | (uint32_t(eb[2]) << 16) | (uint32_t(imask) << 24);
-    o[4] = uint32_t(child_base);
-    o[5] = uint32_t(tri_base);
-    o[6] = pack4(meta); o[7] = pack4(meta + 4);
-    o[8] = pack4(qlo[0]); o[9] = pack4(qlo[0] + 4); o[10] = pack4(qlo[1]); o[11] = pack4(qlo[1] + 4);
-    o[12] = pack4(qlo[2]); o[13] = pack4(qlo[2] + 4); o[14] = pack4(qhi[0]); o[15] = pack4(qhi[0] + 4);
-    o[16] = pack4(qhi[1]); o[17] = pack4(qhi[1] + 4); o[18] = pack4(qhi[2]); o[19] = pack4(qhi[2] + 4);
+}
+
+// Level 0: the root's wide node.
+__global__ void k_emit_start(Emit E) {
+    E.q_bin[0] = E.root->root;
+    E.st->wide_count = 1;
+    E.st->tri_count = 0;
+    E.st->level[0] = 0;
+    E.st->level[1] = 1;
 }
 
 int grid_of(int64_t n) { return int(std::min<int64_t>((n + kBlock - 1) / kBlock, int64_t(1) << 20)); }
@@ -491,119 +725,126 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
     if (n > (int64_t(1) << 30)) throw Error(LMGPU_ERR_UNSUPPORTED, "accel build: more than 2^30 triangles on the GPU builder");
     const size_t nn = size_t(2) * size_t(n);
     const int width = std::min(8, std::max(2, tuning().node_width));
-    DevBuf P, tlo, thi, cen, cb, err, keys[2], vals[2], blo, bhi, bl, br, bc, cost, dec, dnode, cl[2], nnb, flags, scan,
-        totals, q, wide_count, tri_count, tmp;
-    P.alloc(size_t(n) * 36);
-    LMGPU_CUDA(cudaMemcpyAsync(P.p, tri_p, size_t(n) * 36, cudaMemcpyHostToDevice, st));
-    tlo.alloc(size_t(n) * 16); thi.alloc(size_t(n) * 16); cen.alloc(size_t(n) * 16);
-    cb.alloc(6 * 4); err.alloc(4);
-    const uint32_t cb0[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
-    LMGPU_CUDA(cudaMemcpyAsync(cb.p, cb0, sizeof(cb0), cudaMemcpyHostToDevice, st));
-    LMGPU_CUDA(cudaMemsetAsync(err.p, 0, 4, st));
-    const int g = grid_of(n);
-    k_prep<<<g, kBlock, 0, st>>>(P.as<float>(), n, tlo.as<float4>(), thi.as<float4>(), cen.as<float4>(), cb.as<uint32_t>(),
-                                 err.as<int>());
-    for (int b = 0; b < 2; b++) { keys[b].alloc(size_t(n) * 4); vals[b].alloc(size_t(n) * 4); }
-    k_morton<<<g, kBlock, 0, st>>>(cen.as<float4>(), n, cb.as<uint32_t>(), keys[0].as<uint32_t>(), vals[0].as<int32_t>());
-    LMGPU_CUDA(cudaGetLastError());
+    // One allocation holds every temporary (26 of them, with their releases, took most of a small
+    // build's time).
+    size_t sort_bytes = 0;
     {
-        cub::DoubleBuffer<uint32_t> dk(keys[0].as<uint32_t>(), keys[1].as<uint32_t>());
-        cub::DoubleBuffer<int32_t> dv(vals[0].as<int32_t>(), vals[1].as<int32_t>());
-        size_t tb = 0;
-        LMGPU_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dv, int(n), 0, 30, st));
-        tmp.alloc(tb);
-        LMGPU_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, tb, dk, dv, int(n), 0, 30, st));
-        if (dv.Current() != vals[0].as<int32_t>()) {
-            LMGPU_CUDA(cudaMemcpyAsync(vals[0].p, dv.Current(), size_t(n) * 4, cudaMemcpyDeviceToDevice, st));
+        cub::DoubleBuffer<uint32_t> dk(nullptr, nullptr);
+        cub::DoubleBuffer<int32_t> dv(nullptr, nullptr);
+        LMGPU_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, dk, dv, int(n), 0, 30, st));
+    }
+    struct Part {
+        void** p;
+        size_t bytes;
+    };
+    float *P, *cost;
+    float4 *tlo, *thi, *cen, *blo, *bhi;
+    uint32_t *cb, *keys[2];
+    int32_t *vals[2], *bl, *br, *bc, *cl[2], *nnb, *q;
+    int8_t *dec, *dnode;
+    unsigned long long* sums;
+    void* tmp;
+    PlocState* state;
+    RootInfo* root;
+    EmitState* es;
+    auto at = [](auto*& p) { return reinterpret_cast<void**>(&p); };
+    const Part parts[] = {
+        {at(P), size_t(n) * 36}, {at(tlo), size_t(n) * 16}, {at(thi), size_t(n) * 16}, {at(cen), size_t(n) * 16},
+        {at(cb), 24}, {at(keys[0]), size_t(n) * 4}, {at(keys[1]), size_t(n) * 4}, {at(vals[0]), size_t(n) * 4},
+        {at(vals[1]), size_t(n) * 4}, {at(blo), nn * 16}, {at(bhi), nn * 16}, {at(bl), nn * 4}, {at(br), nn * 4},
+        {at(bc), nn * 4}, {at(cost), nn * 32}, {at(dec), nn * 8}, {at(dnode), nn}, {at(cl[0]), size_t(n) * 4},
+        {at(cl[1]), size_t(n) * 4}, {at(nnb), size_t(n) * 4}, {at(sums), (size_t(n) / kBlock + 1) * 8},
+        {at(q), size_t(n) * 4}, {&tmp, sort_bytes}, {at(state), 2 * sizeof(PlocState)},
+        {at(root), sizeof(RootInfo)}, {at(es), sizeof(EmitState)}};
+    size_t total = 0;
+    for (const Part& x : parts) total += (x.bytes + 255) & ~size_t(255);
+    DevBuf arena;
+    arena.alloc(total);
+    {
+        char* p = arena.as<char>();
+        for (const Part& x : parts) {
+            *x.p = p;
+            p += (x.bytes + 255) & ~size_t(255);
         }
     }
-    blo.alloc(nn * 16); bhi.alloc(nn * 16); bl.alloc(nn * 4); br.alloc(nn * 4); bc.alloc(nn * 4);
-    cost.alloc(nn * 8 * 4); dec.alloc(nn * 8); dnode.alloc(nn);
-    Nodes N{blo.as<float4>(), bhi.as<float4>(), bl.as<int32_t>(), br.as<int32_t>(), bc.as<int32_t>(), cost.as<float>(),
-            dec.as<int8_t>(), dnode.as<int8_t>()};
-    cl[0].alloc(size_t(n) * 4); cl[1].alloc(size_t(n) * 4);
-    k_leaves<<<g, kBlock, 0, st>>>(vals[0].as<int32_t>(), n, tlo.as<float4>(), thi.as<float4>(), N, cl[0].as<int32_t>());
+    LMGPU_CUDA(cudaMemcpyAsync(P, tri_p, size_t(n) * 36, cudaMemcpyHostToDevice, st));
+    LMGPU_CUDA(cudaMemsetAsync(cb, 0xff, 12, st));  // ordered minima, then maxima
+    LMGPU_CUDA(cudaMemsetAsync(cb + 3, 0, 12, st));
+    LMGPU_CUDA(cudaMemsetAsync(es, 0, sizeof(EmitState), st));
+    const int g = grid_of(n);
+    k_prep<<<g, kBlock, 0, st>>>(P, n, tlo, thi, cen, cb, &es->err);
+    k_morton<<<g, kBlock, 0, st>>>(cen, n, cb, keys[0], vals[0]);
     LMGPU_CUDA(cudaGetLastError());
-    int hbits = 0;
-    LMGPU_CUDA(cudaMemcpyAsync(&hbits, err.p, 4, cudaMemcpyDeviceToHost, st));
-    LMGPU_CUDA(cudaStreamSynchronize(st));
-    if (hbits & kErrNonFinite) throw Error(LMGPU_ERR_INVALID_ARGUMENT, "accel build: non-finite vertex coordinate");
+    cub::DoubleBuffer<uint32_t> dk(keys[0], keys[1]);
+    cub::DoubleBuffer<int32_t> dv(vals[0], vals[1]);
+    LMGPU_CUDA(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, dk, dv, int(n), 0, 30, st));
+    const Nodes N{blo, bhi, bl, br, bc, cost, dec, dnode};
+    k_leaves<<<g, kBlock, 0, st>>>(dv.Current(), n, tlo, thi, N, cl[0], state);
+    LMGPU_CUDA(cudaGetLastError());
 
-    // PLOC
-    nnb.alloc(size_t(n) * 4); flags.alloc(size_t(n) * 8); scan.alloc(size_t(n) * 8); totals.alloc(8);
-    size_t sb = 0;
-    LMGPU_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, sb, flags.as<unsigned long long>(), scan.as<unsigned long long>(),
-                                             int(n), st));
-    tmp.alloc(sb);
-    int32_t m = int32_t(n), next_id = int32_t(n);
+    int herr = 0;
+    auto check = [&] {
+        if (herr & kErrNonFinite) throw Error(LMGPU_ERR_INVALID_ARGUMENT, "accel build: non-finite vertex coordinate");
+        if (herr & kErrQuantize) throw Error(LMGPU_ERR_INVALID_ARGUMENT, "accel build: box quantization failed");
+        if (herr) throw Error(LMGPU_ERR_INTERNAL, "accel build: internal error (wide node layout)");
+    };
+
+    // PLOC: passes over all clusters, four between two reads of what is left (a pass leaves about three
+    // quarters; blocks past the end leave at once), then the last ones in one block
     int cur = 0, iters = 0;
-    while (m > 1) {
+    for (int32_t m = int32_t(n); m > kLast;) {
         const int gm = int((m + kBlock - 1) / kBlock);
-        k_nearest<<<gm, kBlock, 0, st>>>(cl[cur].as<int32_t>(), m, N.lo, N.hi, nnb.as<int32_t>());
-        k_merge_flags<<<gm, kBlock, 0, st>>>(nnb.as<int32_t>(), m, flags.as<unsigned long long>());
-        LMGPU_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, sb, flags.as<unsigned long long>(), scan.as<unsigned long long>(),
-                                                 m, st));
-        k_merge<<<gm, kBlock, 0, st>>>(cl[cur].as<int32_t>(), m, nnb.as<int32_t>(), flags.as<unsigned long long>(),
-                                       scan.as<unsigned long long>(), next_id, N, cl[1 - cur].as<int32_t>(),
-                                       totals.as<unsigned long long>(), width);
-        LMGPU_CUDA(cudaGetLastError());
-        unsigned long long tot = 0;
-        LMGPU_CUDA(cudaMemcpyAsync(&tot, totals.p, 8, cudaMemcpyDeviceToHost, st));
+        for (int k = 0; k < 4; k++, cur = 1 - cur) {
+            k_nearest<<<gm, kBlock, 0, st>>>(cl[cur], state + cur, N.lo, N.hi, nnb, sums);
+            k_scan_blocks<<<1, 1024, 0, st>>>(sums, gm, state + cur, state + 1 - cur);
+            k_merge<<<gm, kBlock, 0, st>>>(cl[cur], state + cur, nnb, sums, N, cl[1 - cur], width);
+            LMGPU_CUDA(cudaGetLastError());
+        }
+        PlocState h{};
+        LMGPU_CUDA(cudaMemcpyAsync(&h, state + cur, sizeof(h), cudaMemcpyDeviceToHost, st));
+        LMGPU_CUDA(cudaMemcpyAsync(&herr, &es->err, 4, cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaStreamSynchronize(st));
-        const int32_t merges = int32_t(tot >> 32), keep = int32_t(tot & 0xffffffffu);
-        if (merges < 1 || keep != m - merges) throw Error(LMGPU_ERR_INTERNAL, "accel build: clustering made no progress");
-        next_id += merges;
-        m = keep;
-        cur = 1 - cur;
+        check();
+        if (h.m < 1 || h.m >= m || h.next_id - int32_t(n) != int32_t(n) - h.m)
+            throw Error(LMGPU_ERR_INTERNAL, "accel build: clustering made no progress");
+        m = h.m;
         if (++iters > 100000) throw Error(LMGPU_ERR_INTERNAL, "accel build: clustering did not converge");
     }
-    int32_t root = 0;
-    LMGPU_CUDA(cudaMemcpyAsync(&root, cl[cur].p, 4, cudaMemcpyDeviceToHost, st));
-    float rc = 0.f;
-    float4 rlo, rhi;
-    LMGPU_CUDA(cudaMemcpyAsync(&rc, N.cost + size_t(root) * 8, 4, cudaMemcpyDeviceToHost, st));
-    LMGPU_CUDA(cudaMemcpyAsync(&rlo, N.lo + root, 16, cudaMemcpyDeviceToHost, st));
-    LMGPU_CUDA(cudaMemcpyAsync(&rhi, N.hi + root, 16, cudaMemcpyDeviceToHost, st));
-    LMGPU_CUDA(cudaStreamSynchronize(st));
-    {
-        const double dx = double(rhi.x) - rlo.x, dy = double(rhi.y) - rlo.y, dz = double(rhi.z) - rlo.z;
-        const double ra = 2.0 * (dx * dy + dy * dz + dz * dx);
-        sah_cost = ra > 0 ? double(rc) / ra : 0.0;
-    }
+    k_last_passes<<<1, kLast, 0, st>>>(cl[cur], state + cur, N, width, root, &es->err);
+    LMGPU_CUDA(cudaGetLastError());
 
-    // emission, level by level
+    // emission, four levels between two reads of how many nodes there are
     const int32_t cap = int32_t(std::max<int64_t>(n, 1));  // wide nodes never exceed the triangles
     nodes.alloc(size_t(cap) * 80);
     tris.alloc(size_t(n) * 48);
     tri_slot.alloc(size_t(n) * 4);
-    q.alloc(size_t(cap) * 4);
-    wide_count.alloc(4);
-    tri_count.alloc(4);
-    const int32_t one = 1;
-    LMGPU_CUDA(cudaMemcpyAsync(q.p, &root, 4, cudaMemcpyHostToDevice, st));
-    LMGPU_CUDA(cudaMemcpyAsync(wide_count.p, &one, 4, cudaMemcpyHostToDevice, st));
-    LMGPU_CUDA(cudaMemsetAsync(tri_count.p, 0, 4, st));
-    Emit E{N, P.as<float>(), nodes.as<uint32_t>(), tris.as<float4>(), tri_slot.as<int32_t>(), q.as<int32_t>(),
-           wide_count.as<int32_t>(), tri_count.as<int32_t>(), root, cap, err.as<int>(), width};
-    int32_t w0 = 0, w1 = 1, levels = 0;
-    while (w0 < w1) {
-        k_emit<<<int((w1 - w0 + 127) / 128), 128, 0, st>>>(E, w0, w1);
-        LMGPU_CUDA(cudaGetLastError());
-        int32_t nw = 0;
-        LMGPU_CUDA(cudaMemcpyAsync(&nw, wide_count.p, 4, cudaMemcpyDeviceToHost, st));
-        LMGPU_CUDA(cudaMemcpyAsync(&hbits, err.p, 4, cudaMemcpyDeviceToHost, st));
+    const Emit E{N, P, nodes.as<uint32_t>(), tris.as<float4>(), tri_slot.as<int32_t>(), q, es, root, cap, width};
+    k_emit_start<<<1, 1, 0, st>>>(E);
+    LMGPU_CUDA(cudaGetLastError());
+    EmitState h{};
+    int32_t levels = 0;
+    const int emit_grid = int(std::min<int64_t>((n + kEmitBlock / 8 - 1) / (kEmitBlock / 8), int64_t(current_device().num_sms) * 16));
+    auto empty = [&](int32_t l) { return h.level[l & 7] == h.level[(l + 1) & 7]; };
+    do {
+        for (int k = 0; k < 4; k++, levels++) {
+            k_emit<<<emit_grid, kEmitBlock, 0, st>>>(E, levels);
+            LMGPU_CUDA(cudaGetLastError());
+            LMGPU_CUDA(cudaMemcpyAsync(&es->level[(levels + 2) & 7], &es->wide_count, 4, cudaMemcpyDeviceToDevice, st));
+        }
+        LMGPU_CUDA(cudaMemcpyAsync(&h, es, sizeof(h), cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaStreamSynchronize(st));
-        if (hbits & kErrQuantize) throw Error(LMGPU_ERR_INVALID_ARGUMENT, "accel build: box quantization failed");
-        if (hbits) throw Error(LMGPU_ERR_INTERNAL, "accel build: internal error (wide node layout)");
-        levels++;
-        w0 = w1;
-        w1 = nw;
-    }
-    int32_t nt = 0;
-    LMGPU_CUDA(cudaMemcpyAsync(&nt, tri_count.p, 4, cudaMemcpyDeviceToHost, st));
+        herr = h.err;
+        check();
+    } while (!empty(levels));
+    while (levels > 0 && empty(levels - 1)) levels--;
+    if (int64_t(h.tri_count) != n) throw Error(LMGPU_ERR_INTERNAL, "accel build: internal error (triangle count)");
+    RootInfo hr{};
+    LMGPU_CUDA(cudaMemcpyAsync(&hr, root, sizeof(hr), cudaMemcpyDeviceToHost, st));
     LMGPU_CUDA(cudaStreamSynchronize(st));
-    if (int64_t(nt) != n) throw Error(LMGPU_ERR_INTERNAL, "accel build: internal error (triangle count)");
-    num_nodes = w1;
+    const double dx = double(hr.hi[0]) - hr.lo[0], dy = double(hr.hi[1]) - hr.lo[1], dz = double(hr.hi[2]) - hr.lo[2];
+    const double ra = 2.0 * (dx * dy + dy * dz + dz * dx);
+    sah_cost = ra > 0 ? double(hr.cost) / ra : 0.0;
+    num_nodes = h.wide_count;
     depth = levels;
 }
 
