@@ -340,7 +340,8 @@ typedef struct lmgpu_render_stats {
     int64_t shadow_rays;
     double elapsed_ms;          /* device time of the render (CUDA events) */
     double trace_ms;            /* device time inside the extension + shadow trace kernels */
-    double extend_ms, shade_ms, shadow_ms, generate_ms;  /* device time per kernel kind */
+    double extend_ms, shade_ms, shadow_ms, generate_ms;  /* device time per kernel kind (shadow launches may run
+                                                            beside extension launches: both count in full) */
     int64_t extend_launches, shadow_launches;
     /* with params->instrument: mean 8-wide nodes visited / triangles tested per traced ray */
     double ext_nodes, ext_tris, shadow_nodes, shadow_tris;
@@ -461,7 +462,7 @@ int lmgpu_batch_resolve(lmgpu_batch* batch, int32_t job, void* stream);
 int lmgpu_batch_get_stats(const lmgpu_batch* batch, lmgpu_render_stats* out);
 /* Forgets every job (buffers stay allocated). */
 int lmgpu_batch_reset(lmgpu_batch* batch);
-/* on != 0: runs also time every kernel (event nodes in the captured chunk); lmgpu_batch_get_stats
+/* on != 0: runs also time every kernel (time stamps taken by the kernels); lmgpu_batch_get_stats
  * then reports extend_ms, shade_ms, shadow_ms and generate_ms (planner + camera vertices). */
 int lmgpu_batch_set_timing(lmgpu_batch* batch, int32_t on);
 

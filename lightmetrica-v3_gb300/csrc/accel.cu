@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(Bvh8 bvh, const flo
         if (threadIdx.x == 0) s_fetch = 0;
         __syncthreads();
         fetch_loop<kAnyHit, false, kTwoLevel>(
-            int(count), int(blockDim.x / 32), Fetch{&s_fetch, nullptr, refill}, stk, stride, &lerr,
+            int(count), int(blockDim.x / 32), Fetch{&s_fetch, {nullptr, nullptr}, refill, nullptr, nullptr}, stk, stride, &lerr,
             [&](int k, Trav& s) {
                 const int64_t i = ray_of(k);
                 const float4 a = rays[2 * i], b = rays[2 * i + 1];

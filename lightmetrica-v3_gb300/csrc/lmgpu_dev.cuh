@@ -423,15 +423,39 @@ __device__ inline TraceHit trace_bvh8(const Bvh8& bvh, f3 o, f3 d, float tmin, f
     return s.best;
 }
 
+__device__ inline unsigned long long globaltimer_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 // Dynamic ray fetch for the persistent trace kernels: `self` hands out queue entries (zero at
-// launch); `other`, when set, is the counter of another trace kernel that this launch resets for
-// that kernel's next launch (the path tracers' extension and shadow kernels alternate on one
-// stream, so neither counter is in use while the other kernel runs). refill: see Tuning.
+// launch). The launch zeroes the counters in `reset` (where set) at its start, for kernels that run
+// after it and that no kernel in flight uses. refill: see Tuning. With `stamp`, the launch writes its
+// start and end times there ([0], [1], in ns); `done` counts its finished blocks (zero between
+// launches).
 struct Fetch {
     int* self;
-    int* other;
+    int* reset[2];
     int refill;
+    unsigned long long* stamp;
+    int* done;
 };
+__device__ __forceinline__ void trace_begin(const Fetch& f) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    if (f.reset[0]) *f.reset[0] = 0;
+    if (f.reset[1]) *f.reset[1] = 0;
+    if (f.stamp) f.stamp[0] = globaltimer_ns();
+}
+// Called by all threads of the block at the launch's end.
+__device__ __forceinline__ void trace_end(const Fetch& f) {
+    if (!f.stamp) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(f.done, 1) == int(gridDim.x) - 1) {
+        *f.done = 0;
+        f.stamp[1] = globaltimer_ns();
+    }
+}
 
 // Cooperative traversal: eight lanes per ray, four rays per warp, for launches and queue ends that
 // leave fewer rays than lanes. A lane tests one child box and one triangle, so a visit takes about

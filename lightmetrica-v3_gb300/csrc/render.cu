@@ -809,9 +809,8 @@ __device__ inline void nee(const DevScene& S, const PtConst& P, const Geom& g, c
 }
 
 template <bool kBatched>
-__device__ inline void push_ext(const ExtQ& q, int* count, f3 o, f3 d, f3 thr, float pdf, f3 n, uint32_t flags, uint32_t path,
-                                uint32_t pixel, uint32_t job) {
-    const int k = queue_slot(count);
+__device__ inline void store_ext(const ExtQ& q, int64_t k, f3 o, f3 d, f3 thr, float pdf, f3 n, uint32_t flags, uint32_t path,
+                                 uint32_t pixel, uint32_t job) {
     q.o[k] = make_float4(o.x, o.y, o.z, 0.f);
     q.d[k] = make_float4(d.x, d.y, d.z, 0.f);
     q.thr[k] = make_float4(thr.x, thr.y, thr.z, pdf);
@@ -819,13 +818,31 @@ __device__ inline void push_ext(const ExtQ& q, int* count, f3 o, f3 d, f3 thr, f
     q.ids[k] = make_uint2(path, pixel);
     if (kBatched) q.job[k] = job;
 }
+template <bool kBatched>
+__device__ inline void push_ext(const ExtQ& q, int* count, f3 o, f3 d, f3 thr, float pdf, f3 n, uint32_t flags, uint32_t path,
+                                uint32_t pixel, uint32_t job) {
+    store_ext<kBatched>(q, queue_slot(count), o, d, thr, pdf, n, flags, path, pixel, job);
+}
+
+// Counters that a shade launch zeroes at its start (where set), for kernels that run after it and
+// that no kernel in flight uses; `stamp` receives its start time (ns).
+struct Resets {
+    int* p[3];
+    unsigned long long* stamp;
+};
+__device__ __forceinline__ void reset_counters(const Resets& r) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    for (int i = 0; i < 3; i++)
+        if (r.p[i]) *r.p[i] = 0;
+    if (r.stamp) *r.stamp = globaltimer_ns();
+}
 
 // Camera vertex of one path: renderer_pt.cpp:95-116 and the first pass of the loop (NEE in image
 // mode, the jittered primary direction, raster position caching). `path` is the RNG key
-// pixel * spp + sample; `pix` the pixel whose window is sampled.
+// pixel * spp + sample; `pix` the pixel whose window is sampled; `slot` its entry in the queue.
 template <bool kBatched>
 __device__ __forceinline__ void generate_path(const DevScene& S, const PtConst& P, uint64_t path, int64_t pix, const ExtQ& q,
-                                              int* qcount, const ShadowQ& sq, int* scount, uint32_t job, uint32_t odd_bit) {
+                                              int64_t slot, const ShadowQ& sq, int* scount, uint32_t job, uint32_t odd_bit) {
     float wx = 0.f, wy = 0.f, ww = 1.f, wh = 1.f;
     if (!P.image) {
         const int x = int(pix % P.w), y = int(pix / P.w);
@@ -846,17 +863,18 @@ __device__ __forceinline__ void generate_path(const DevScene& S, const PtConst& 
     raster_pos(S, d, rx, ry);
     const uint32_t pixel = pixel_of(P, rx, ry);
     const float pdf = nee_ok ? cam_pdf(S, d) : 0.f;
-    push_ext<kBatched>(q, qcount, S.cam_p, d, mk(1, 1, 1), pdf, mk(0, 0, 0), (nee_ok ? 1u : 0u) | 2u | (1u << 8),
-                       uint32_t(path), pixel, job);
+    store_ext<kBatched>(q, slot, S.cam_p, d, mk(1, 1, 1), pdf, mk(0, 0, 0), (nee_ok ? 1u : 0u) | 2u | (1u << 8),
+                        uint32_t(path), pixel, job);
 }
 
 // Single scene: paths [start, start + count) enumerated pixel-major (path = pixel * spp + sample).
 __global__ void __launch_bounds__(kBlock) k_pt_generate(const __grid_constant__ DevScene S, const __grid_constant__ PtConst P,
                                                         int64_t start, int64_t count, ExtQ q, int* qcount, ShadowQ sq,
                                                         int* scount) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *qcount = int(count);
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
         const uint64_t path = uint64_t(start + i);
-        generate_path<false>(S, P, path, int64_t(path / uint64_t(P.spp)), q, qcount, sq, scount, 0u, 0u);
+        generate_path<false>(S, P, path, int64_t(path / uint64_t(P.spp)), q, i, sq, scount, 0u, 0u);
     }
 }
 
@@ -873,25 +891,60 @@ struct ActiveJob {
     int32_t job, pad;
 };
 
-// New paths for the slots the planner handed out this iteration (ctl[3] of them, in ctl[22]
-// allocation entries; both read here, not baked into a captured launch).
+// New paths, behind the queue's *survivors* entries; *qn becomes the queue's length. One job
+// (kSingle): every block plans for itself, as many of the job's next paths as the queue has room for
+// (`started` paths before the launch, next[0] after it), so an iteration needs no planner launch.
+// Job table: the slots the planner handed out (ctl[3] of them, in ctl[22] allocation entries). What
+// the kernel reads is written by none of its blocks, and everything comes from device memory, not
+// baked into a captured launch.
+struct GenState {
+    const int64_t* started;  // one job: paths started before this launch
+    int64_t* next;           // one job: after it
+    int64_t* job_next;       // one job: the planner's count, kept for jobs that join later
+    int64_t cap;
+    const int* survivors;
+    int* qn;
+    unsigned long long* stamp;
+};
+template <bool kSingle>
 __global__ void __launch_bounds__(kBlock) k_wf_generate(const JobDev* __restrict__ jobs, const AllocEntry* __restrict__ alloc,
-                                                        const int64_t* __restrict__ ctl, ExtQ q, int* qcount, ShadowQ sq,
+                                                        const int64_t* __restrict__ ctl, GenState G, ExtQ q, ShadowQ sq,
                                                         int* scount) {
-    const int64_t count = ctl[3];
-    const int na = int(ctl[22]);
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
-        int lo = 0, hi = na;  // last entry with slot <= i
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (alloc[mid].slot <= i) lo = mid; else hi = mid;
+    const int64_t inq = *G.survivors;
+    int64_t count, started = 0;
+    int na = 0;
+    if (kSingle) {
+        started = *G.started;
+        count = max(int64_t(0), min(G.cap - inq, jobs[0].limit - started));
+    } else {
+        count = ctl[3];
+        na = int(ctl[22]);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *G.qn = int(inq + count);
+        if (kSingle) {
+            *G.next = started + count;
+            *G.job_next = started + count;
         }
-        const AllocEntry e = alloc[lo];
-        const JobDev& J = jobs[e.job];
-        const int64_t local = e.local + (i - e.slot);
+        if (G.stamp) *G.stamp = globaltimer_ns();
+    }
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
+        int32_t job = 0;
+        int64_t local = started + i;
+        if (!kSingle) {
+            int lo = 0, hi = na;  // last entry with slot <= i
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (alloc[mid].slot <= i) lo = mid; else hi = mid;
+            }
+            const AllocEntry e = alloc[lo];
+            job = e.job;
+            local = e.local + (i - e.slot);
+        }
+        const JobDev& J = jobs[job];
         const int64_t sample = local / J.npix, pix = local - sample * J.npix;
         const uint32_t odd = (J.film_odd && ((uint32_t(sample) + J.parity0) & 1u)) ? kOddPass : 0u;
-        generate_path<true>(J.S, J.P, uint64_t(pix * J.P.spp + sample), pix, q, qcount, sq, scount, uint32_t(e.job), odd);
+        generate_path<true>(J.S, J.P, uint64_t(pix * J.P.spp + sample), pix, q, inq + i, sq, scount, uint32_t(job), odd);
     }
 }
 
@@ -920,10 +973,8 @@ __global__ void __launch_bounds__(kTrace, kExtendBlocks) k_pt_extend(Bvh8 bvh, c
                                                       const uint32_t* __restrict__ qjob = nullptr) {
     extern __shared__ uint2 smem[];
     const int n = *qcount;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(rays, (unsigned long long)n);
-        if (f.other) *f.other = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(rays, (unsigned long long)n);
+    trace_begin(f);
     uint2* stk = smem + threadIdx.x;
     int lerr = 0;
     uint32_t cn = 0, ct = 0, cc = 0;
@@ -969,6 +1020,7 @@ __global__ void __launch_bounds__(kTrace, kExtendBlocks) k_pt_extend(Bvh8 bvh, c
         atomicAdd(sums + 2, (unsigned long long)cc);
     }
     if (lerr) atomicOr(err, lerr);
+    trace_end(f);
 }
 
 // Shadow rays: any hit over [Eps, tmax]; unoccluded contributions go to the film. kCount,
@@ -985,10 +1037,8 @@ __global__ void __launch_bounds__(kTrace, kShadowBlocks) k_pt_shadow(Bvh8 bvh, S
         if (pw & kOddPass) return kBatched ? jobs[job].film_odd : film_odd;
         return kBatched ? jobs[job].film : film;
     };
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        atomicAdd(rays, (unsigned long long)n);
-        if (f.other) *f.other = 0;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(rays, (unsigned long long)n);
+    trace_begin(f);
     uint2* stk = smem + threadIdx.x;
     int lerr = 0;
     uint32_t cn = 0, ct = 0, cc = 0;
@@ -1043,6 +1093,7 @@ __global__ void __launch_bounds__(kTrace, kShadowBlocks) k_pt_shadow(Bvh8 bvh, S
         atomicAdd(sums + 5, (unsigned long long)cc);
     }
     if (lerr) atomicOr(err, lerr);
+    trace_end(f);
 }
 
 // One pass of the loop body after the intersection (renderer_pt.cpp:221-300) for one path whose
@@ -1182,8 +1233,9 @@ __global__ void __launch_bounds__(kBlock) k_lt_generate(const __grid_constant__ 
 template <int kMinBlocks, uint32_t kF = kFeatAll>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) k_lt_shade(const __grid_constant__ DevScene S, const __grid_constant__ PtConst P,
                                                      ExtQ qi, const float4* __restrict__ hits, const int* __restrict__ qicount,
-                                                     ExtQ qo, int* qocount, ShadowQ sq, int* scount) {
+                                                     ExtQ qo, int* qocount, ShadowQ sq, int* scount, Resets resets) {
     const int n = *qicount;
+    reset_counters(resets);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const float4 h4 = hits[k];
         const int32_t id = __float_as_int(h4.w);
@@ -1415,8 +1467,9 @@ __global__ void __launch_bounds__(kBlock) k_bd_generate(const __grid_constant__ 
 template <int kMinBlocks, uint32_t kF = kFeatAll>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) k_bd_shade(const __grid_constant__ DevScene S, const __grid_constant__ PtConst P,
                                                      BdRec R, ExtQ qi, const float4* __restrict__ hits, const int* __restrict__ qicount,
-                                                     ExtQ qo, int* qocount) {
+                                                     ExtQ qo, int* qocount, Resets resets) {
     const int n = *qicount;
+    reset_counters(resets);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const float4 h4 = hits[k], o4 = qi.o[k], d4 = qi.d[k], t4 = qi.thr[k], n4 = qi.nrm[k];
         const uint2 ids = qi.ids[k];
@@ -1792,8 +1845,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_bd_connect(const __grid_
 template <int kMinBlocks, bool kSingle, uint32_t kF = kFeatAll>
 __global__ void __launch_bounds__(kBlock, kMinBlocks) k_wf_shade(const JobDev* __restrict__ jobs, ExtQ qi, const float4* __restrict__ hits,
                                                      const int* __restrict__ qicount, ExtQ qo, int* qocount, ShadowQ sq,
-                                                     int* scount, unsigned int* pass_done) {
+                                                     int* scount, unsigned int* pass_done, Resets resets) {
     const int n = *qicount;
+    reset_counters(resets);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         // kSingle: the batch holds one job, so no per-path job id is read
         const uint32_t job = kSingle ? 0u : qi.job[k];
@@ -1821,8 +1875,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_wf_shade(const JobDev* _
 // out, [4] paths in flight or waiting (0 = done), [5] jobs submitted, [20] jobs seen, [21]
 // active jobs, [22] allocation entries.
 __global__ void __launch_bounds__(32) k_wf_plan(int64_t* ctl, const int* qcount, int64_t cap, const JobDev* __restrict__ jobs,
-                                                int64_t* job_next, ActiveJob* active, AllocEntry* alloc, int first_pass) {
+                                                int64_t* job_next, ActiveJob* active, AllocEntry* alloc, int first_pass,
+                                                unsigned long long* stamp) {
     const int lane = int(threadIdx.x);
+    if (stamp && lane == 0) *stamp = globaltimer_ns();
     const unsigned below = (1u << lane) - 1u;
     const int64_t njobs = ctl[5], seen = ctl[20];
     int64_t nact = ctl[21];
@@ -2003,6 +2059,16 @@ struct Workspace {
     DevBuf q_o[2], q_d[2], q_thr[2], q_nrm[2], q_ids[2], hits, s_o, s_d, s_c, counters;
     lmgpu_batch* batch = nullptr;  // the regenerating wavefront lmgpu_render_pt runs its job on
     int64_t batch_cap = 0;
+    // stream of the shadow rays that run beside the next bounce's extension rays, and the events that
+    // order the two (created on first use)
+    cudaStream_t side = nullptr;
+    cudaEvent_t shaded = nullptr, shadowed = nullptr;
+    void ensure_side() {
+        if (side) return;
+        LMGPU_CUDA(cudaEventCreateWithFlags(&shaded, cudaEventDisableTiming));
+        LMGPU_CUDA(cudaEventCreateWithFlags(&shadowed, cudaEventDisableTiming));
+        LMGPU_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+    }
     DevBuf bd_rec, bd_nv, bd_s_o, bd_s_d, bd_s_c, bd_items, bd_items_sorted, bd_hist;  // lmgpu_render_bdpt: subpath records,
     // connection rays, strategies (and in strategy-major order), the sort's bucket counts
 };
@@ -2590,7 +2656,7 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
         // [0],[1] extension queues, [2] shadow queue, [3] error, [4],[5] extension / shadow ray fetch
         int* cnt = ws.counters.as<int>();
         const int refill = tuning().trace_refill;
-        const Fetch f_ext{cnt + 4, cnt + 5, refill}, f_sh{cnt + 5, cnt + 4, refill};
+        const Fetch f_ext{cnt + 4, {cnt + 5, nullptr}, refill, nullptr, nullptr}, f_sh{cnt + 5, {cnt + 4, nullptr}, refill, nullptr, nullptr};
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
@@ -2798,10 +2864,11 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
             q[b] = ExtQ{ws.q_o[b].as<float4>(), ws.q_d[b].as<float4>(), ws.q_thr[b].as<float4>(), ws.q_nrm[b].as<float4>(),
                         ws.q_ids[b].as<uint2>()};
         ShadowQ sq{ws.s_o.as<float4>(), ws.s_d.as<float4>(), ws.s_c.as<float4>()};
-        // [0],[1] extension queues, [2] shadow queue, [3] error, [4],[5] extension / shadow ray fetch
+        // [0],[1] extension queues, [2],[6] shadow rays of even and odd bounces, [3] error, [4],[5] extension
+        // and shadow ray fetch
         int* cnt = ws.counters.as<int>();
         const int refill = tuning().trace_refill;
-        const Fetch f_ext{cnt + 4, cnt + 5, refill}, f_sh{cnt + 5, cnt + 4, refill};
+        ws.ensure_side();
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
@@ -2820,11 +2887,11 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
         enum { K_GEN = 0, K_EXT = 1, K_SHADE = 2, K_SHADOW = 3 };
         std::vector<std::pair<int, cudaEvent_t>> marks;
         const bool timed = stats != nullptr;
-        auto mark = [&](int kind) {
+        auto mark = [&](int kind, cudaStream_t on = nullptr) {
             if (!timed) return;
             cudaEvent_t e;
             LMGPU_CUDA(cudaEventCreate(&e));
-            LMGPU_CUDA(cudaEventRecord(e, st));
+            LMGPU_CUDA(cudaEventRecord(e, on ? on : st));
             marks.emplace_back(kind, e);
         };
         cudaEvent_t e0, e1;
@@ -2845,33 +2912,43 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
             const int64_t n = std::min(wave, total - start);
             int cur = 0;
             LMGPU_CUDA(cudaMemsetAsync(cnt, 0, 12, st));
-            LMGPU_CUDA(cudaMemsetAsync(cnt + 4, 0, 8, st));
+            LMGPU_CUDA(cudaMemsetAsync(cnt + 4, 0, 12, st));
             mark(K_GEN);
             k_lt_generate<<<int(std::min<int64_t>(g_gen, (n + kBlock - 1) / kBlock)), kBlock, 0, st>>>(
                 s->dev, P, prm->first_path + start, n, q[0], cnt + 0);
             mark(-1);
             LMGPU_CUDA(cudaGetLastError());
-            // the ray that leaves vertex it; its hit connects when it + 1 < max_verts
+            // The ray that leaves vertex it; its hit connects when it + 1 < max_verts. A bounce's shadow
+            // rays run beside the next bounce's extension rays: each launch ends with some 100 us in which
+            // its longest rays run alone, and of the two kinds' only one is waited for (frame of 2^22 light
+            // paths 4.67 -> 4.32 ms). Shade, which fills the shadow queue again, waits for both. The
+            // counters are zeroed by launches that none of their users runs beside, not by memsets.
             for (int it = 1; it + 1 < P.max_verts; it++) {
+                int *sc = cnt + (it & 1 ? 2 : 6), *sc_next = cnt + (it & 1 ? 6 : 2);
+                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, nullptr, nullptr};
+                const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, nullptr, nullptr};
                 mark(K_EXT);
                 ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
                 mark(-1);
                 n_ext++;
-                LMGPU_CUDA(cudaMemsetAsync(cnt + (1 - cur), 0, 4, st));
-                LMGPU_CUDA(cudaMemsetAsync(cnt + 2, 0, 4, st));
+                if (it > 1) LMGPU_CUDA(cudaStreamWaitEvent(st, ws.shadowed, 0));
                 mark(K_SHADE);
                 shade_k<<<g_shade, kBlock, 0, st>>>(s->dev, P, q[cur], ws.hits.as<float4>(), cnt + cur, q[1 - cur], cnt + (1 - cur),
-                                                      sq, cnt + 2);
+                                                      sq, sc, Resets{{cnt + 4, cnt + 5, sc_next}, nullptr});
                 mark(-1);
-                mark(K_SHADOW);
-                sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr,
-                                                  nullptr);
-                mark(-1);
+                LMGPU_CUDA(cudaEventRecord(ws.shaded, st));
+                LMGPU_CUDA(cudaStreamWaitEvent(ws.side, ws.shaded, 0));
+                mark(K_SHADOW, ws.side);
+                sh_k<<<g_sh, kTrace, tsmem, ws.side>>>(bvh, sq, sc, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr,
+                                                       nullptr);
+                mark(-1, ws.side);
+                LMGPU_CUDA(cudaEventRecord(ws.shadowed, ws.side));
                 n_sh++;
                 LMGPU_CUDA(cudaGetLastError());
                 cur = 1 - cur;
             }
+            if (P.max_verts > 2) LMGPU_CUDA(cudaStreamWaitEvent(st, ws.shadowed, 0));
         }
         f->accumulated_spp += total;
         const double scale = double(npix) / double(f->accumulated_spp);
@@ -2977,7 +3054,7 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
         // [0],[1] extension queues, [2] connection rays, [3] error, [4],[5] ray fetch, [6] strategies
         int* cnt = ws.counters.as<int>();
         const int refill = tuning().trace_refill;
-        const Fetch f_ext{cnt + 4, cnt + 5, refill}, f_sh{cnt + 5, cnt + 4, refill};
+        const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, nullptr, nullptr};
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
@@ -3032,17 +3109,16 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
             LMGPU_CUDA(cudaGetLastError());
             // the ray that leaves subpath vertex it creates vertex it + 1 (at most max_verts - 1)
             for (int it = 0; it + 1 < mv; it++) {
-                // the extend kernel's fetch counter is otherwise reset by the shadow kernel, which
-                // runs once per wave here
-                LMGPU_CUDA(cudaMemsetAsync(cnt + 4, 0, 4, st));
+                // the shade kernel zeroes the fetch counter for the next bounce's launch
+                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, nullptr, nullptr};
                 mark(K_EXT);
                 ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
                 mark(-1);
                 n_ext++;
-                LMGPU_CUDA(cudaMemsetAsync(cnt + (1 - cur), 0, 4, st));
                 mark(K_SHADE);
-                shade_k<<<g_shade, kBlock, 0, st>>>(s->dev, P, R, q[cur], ws.hits.as<float4>(), cnt + cur, q[1 - cur], cnt + (1 - cur));
+                shade_k<<<g_shade, kBlock, 0, st>>>(s->dev, P, R, q[cur], ws.hits.as<float4>(), cnt + cur, q[1 - cur], cnt + (1 - cur),
+                                                    Resets{{cnt + 4, nullptr, nullptr}, nullptr});
                 mark(-1);
                 LMGPU_CUDA(cudaGetLastError());
                 cur = 1 - cur;
@@ -3181,7 +3257,7 @@ int lmgpu_render_pt_noalloc(lmgpu_scene* s, float* d_film, int32_t w, int32_t h,
         // [0],[1] extension queues, [2] shadow queue, [3] error, [4],[5] extension / shadow ray fetch
         int* cnt = reinterpret_cast<int*>(base);
         const int refill = tuning().trace_refill;
-        const Fetch f_ext{cnt + 4, cnt + 5, refill}, f_sh{cnt + 5, cnt + 4, refill};
+        const Fetch f_ext{cnt + 4, {cnt + 5, nullptr}, refill, nullptr, nullptr}, f_sh{cnt + 5, {cnt + 4, nullptr}, refill, nullptr, nullptr};
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(base + 32);
         unsigned long long* sums = reinterpret_cast<unsigned long long*>(base + 64);
         char* p = base + kNoallocCounters;
@@ -3291,13 +3367,14 @@ struct lmgpu_batch {
     uint32_t passes = 0;
     bool table_dirty = false;
     int32_t max_depth = 1;
-    // captured chunk of iterations: [0] plain, [1] with event nodes between the kernels
+    // captured chunk of iterations: [0] plain, [1] with the kernels' time stamps
     struct GraphSlot {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         int32_t depth = 0;
         int refill = -1, shade = -1, first_pass = -1, specialize = -1;
-        bool two_level = false;
+        bool two_level = false, image = false;
+        int iters = 0;
         bool single = false;      // captured for a one-job table
         uint32_t feat = 0;        // that job's scene features (the shade kernel specialised for them)
         lmgpu::Bvh8 bvh{};        // that job's tree and films, passed by value to the trace kernels
@@ -3313,31 +3390,47 @@ struct lmgpu_batch {
     int refill = 0, shade_minblocks = 3, first_pass = 1, specialize = 1;
     bool two_level = false;  // some job's scene is instanced
     bool timed = false;      // per-kernel device time (lmgpu_batch_set_timing)
-    cudaEvent_t ev[6 * 8] = {};
+    cudaEvent_t e0 = nullptr, e1 = nullptr;  // around a run
+    bool image = false;      // some job samples primary rays over the image (its generate launches queue shadow rays)
     double kms[4] = {0, 0, 0, 0};  // extend, shade, shadow, plan + generate
-    int64_t chunks_run = 0;
+    int64_t iters_run = 0;
     double elapsed_ms = 0;
     ~lmgpu_batch() {
         slot[0].clear();
         slot[1].clear();
-        for (auto& e : ev)
-            if (e) cudaEventDestroy(e);
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
     }
 };
 
 namespace lmgpu {
 namespace {
 
-constexpr int kChunkIters = 8;  // even: the queue parity is the same at every chunk boundary
+constexpr int kChunkIters = 8;      // even: the queue parity is the same at every chunk boundary
+constexpr int kMaxChunkIters = 16;  // longest chunk (one job whose paths all start at once)
 
-// ctl layout (bytes): 0 next, 8 total, 16 range start, 24 range count, 32 remaining, 40 njobs,
-// 48 int counters [0],[1] extension queues, [2] shadow queue, [3] error; 64 u64 rays [2];
-// 80 u64 sums [8]; 144 int extension / shadow ray fetch
+// Stamps of one iteration (ns): launches' start times, and the trace launches' ends.
+struct IterStamps {
+    unsigned long long gen, ext[2], shade, shadow[2];
+};
+// Control words. The planner indexes the first 32 as int64 (its comment); the rest are counters, each
+// written only by launches that none of its readers runs beside.
+struct Ctl {
+    int64_t started, total, pad2, slots, left, njobs;  // [0]..[5]; left: paths in flight or not started
+    int survivors[2];                                  // extension queue entries after shade (per queue)
+    int shadow_even, err;                              // shadow rays of even iterations; error code
+    unsigned long long rays[2], sums[8];
+    int fetch[2], qn[2];                               // ray fetch; queue lengths after generate
+    int64_t seen, active, allocs;                      // [20]..[22]
+    int shadow_odd, done[2], pad3;                     // finished blocks of the timed trace launches
+    int64_t started_odd;
+    unsigned long long end;                            // start of the launch after the last iteration
+    IterStamps it[kMaxChunkIters];
+};
+static_assert(offsetof(Ctl, survivors) == 48 && offsetof(Ctl, rays) == 64 && offsetof(Ctl, fetch) == 144 && offsetof(Ctl, seen) == 160,
+              "the planner, lmgpu_batch_job_set_spp and the statistics index the control words");
+Ctl* ctl_of(const lmgpu_batch* b) { return b->ctl.as<Ctl>(); }
 int64_t* ctl64(lmgpu_batch* b) { return b->ctl.as<int64_t>(); }
-int* ctl_cnt(lmgpu_batch* b) { return reinterpret_cast<int*>(b->ctl.as<char>() + 48); }
-unsigned long long* ctl_rays(lmgpu_batch* b) { return reinterpret_cast<unsigned long long*>(b->ctl.as<char>() + 64); }
-unsigned long long* ctl_sums(lmgpu_batch* b) { return reinterpret_cast<unsigned long long*>(b->ctl.as<char>() + 80); }
-int* ctl_fetch(lmgpu_batch* b) { return reinterpret_cast<int*>(b->ctl.as<char>() + 144); }
 
 // Appends v[done, size) to the device copy (all of v after a reallocation); `done` becomes size.
 template <typename T>
@@ -3361,7 +3454,10 @@ void grow_upload(DevBuf& buf, size_t& cap, size_t& done, const std::vector<T>& v
 }
 
 // paths in flight (the queue the next iteration starts from) plus paths not started yet
-__global__ void k_wf_left(int64_t* ctl, const int* qcount) { ctl[4] = int64_t(*qcount) + (ctl[1] - ctl[0]); }
+__global__ void k_wf_left(Ctl* c, int cur, int timed) {
+    c->left = int64_t(c->survivors[cur]) + (c->total - c->started);
+    if (timed) c->end = globaltimer_ns();
+}
 
 __global__ void k_wf_set_total(int64_t* ctl, int64_t total, int64_t njobs) {
     ctl[1] = total;
@@ -3402,8 +3498,17 @@ uint32_t table_features(const lmgpu_batch* b) {
     return f;
 }
 
-// Stream-ordered view of one chunk of iterations; captured into a graph.
-void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, bool timed) {
+// Bounce iterations of a chunk: eight, or for one job whose paths all start at once and that runs to
+// its end as many as its longest path has bounces (at most 16).
+int chunk_iters(const lmgpu_batch* b, bool to_end) {
+    if (!to_end || b->host_jobs.size() != 1 || b->host_jobs[0].limit > b->cap) return kChunkIters;
+    const int n = b->host_jobs[0].P.max_verts - 1;
+    return std::min(kMaxChunkIters, std::max(2, n + (n & 1)));
+}
+
+// Stream-ordered view of one chunk of iterations; captured into a graph. `side`: a second stream of
+// the capture, with events `shaded` and `shadowed` between the two.
+void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent_t shaded, cudaEvent_t shadowed, bool timed, int iters) {
     const size_t tsmem = size_t(2) * 4 * kTrace * size_t(b->max_depth);
     Bvh8 bmax{};
     bmax.depth = b->max_depth;
@@ -3420,14 +3525,15 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, bool timed) {
     const int g_sh = grid_for(sh_k, kTrace, tsmem);
     auto shade_k = wf_shade_kernel(b, single, table_features(b));
     const int g_shade = grid_for(shade_k, kBlock, 0);
-    const int g_gen = grid_for(k_wf_generate, kBlock, 0);
+    auto gen_k = single ? k_wf_generate<true> : k_wf_generate<false>;
+    const int g_gen = grid_for(gen_k, kBlock, 0);
     Bvh8 tb = bmax;  // stack sized by the deepest tree seen; single job: its own tree
     if (single) {
         tb = J0.S.bvh;
         tb.depth = b->max_depth;
     }
     float* sfilm = single ? J0.film : nullptr;
-    int* cnt = ctl_cnt(b);
+    Ctl* c = ctl_of(b);
     const JobDev* jobs = b->jobs.as<JobDev>();
     ExtQ q[2];
     for (int i = 0; i < 2; i++)
@@ -3435,41 +3541,48 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, bool timed) {
                     b->q_ids[i].as<uint2>(), b->q_job[i].as<uint32_t>()};
     ShadowQ sq{b->s_o.as<float4>(), b->s_d.as<float4>(), b->s_c.as<float4>(), b->s_job.as<uint32_t>()};
     float4* hits = b->hits.as<float4>();
-    int* fetch = ctl_fetch(b);
-    const Fetch f_ext{fetch, fetch + 1, b->refill}, f_sh{fetch + 1, fetch, b->refill};
-    // timed: event record nodes between the kernels, read after each chunk (ev[6*it + k])
-    auto mark = [&](int it, int k) {
-        if (timed) LMGPU_CUDA(cudaEventRecordWithFlags(b->ev[6 * it + k], st, cudaEventRecordExternal));
-    };
     // One bounce iteration: top the queue up with new paths (plan, generate), trace it (extend),
-    // shade the hits into the other queue and the shadow queue, trace the shadow rays.
+    // shade the hits into the other queue and the shadow queue, trace the shadow rays. The shadow rays
+    // run beside the next iteration up to its shade launch, which fills their queue again (so the tail
+    // of a trace launch, in which its longest rays run alone, is waited for once per iteration); with
+    // image-mode jobs, whose generate launches add shadow rays, up to the next iteration. Counters are
+    // zeroed by launches that none of their users runs beside, time stamps are taken by the kernels: an
+    // iteration of one job is four launches (five, two memsets and five event nodes before; a 64x64
+    // preview of 4 spp 520 -> 288 us, the 1080p frame at 16 spp 31.7 -> 28.4 ms).
     int cur = 0;
-    for (int it = 0; it < kChunkIters; it++) {
-        mark(it, 0);
-        k_wf_plan<<<1, 32, 0, st>>>(ctl64(b), cnt + cur, b->cap, jobs, b->job_next.as<int64_t>(), b->active.as<ActiveJob>(),
-                                    b->alloc.as<AllocEntry>(), b->first_pass);
-        k_wf_generate<<<g_gen, kBlock, 0, st>>>(jobs, b->alloc.as<AllocEntry>(), ctl64(b), q[cur], cnt + cur, sq, cnt + 2);
-        mark(it, 1);
-        ext_k<<<g_ext, kTrace, tsmem, st>>>(tb, q[cur].o, q[cur].d, cnt + cur, hits, ctl_rays(b), cnt + 3, ctl_sums(b), 63,
-                                            nullptr, f_ext, single ? nullptr : jobs, single ? nullptr : q[cur].job);
-        mark(it, 2);
-        LMGPU_CUDA(cudaMemsetAsync(cnt + (1 - cur), 0, sizeof(int), st));
-        shade_k<<<g_shade, kBlock, 0, st>>>(jobs, q[cur], hits, cnt + cur, q[1 - cur], cnt + (1 - cur), sq, cnt + 2,
-                                            b->pass_done.as<unsigned int>());
-        mark(it, 3);
-        sh_k<<<g_sh, kTrace, tsmem, st>>>(tb, sq, cnt + 2, sfilm, ctl_rays(b) + 1, cnt + 3, ctl_sums(b), 63, nullptr, f_sh,
-                                          single ? nullptr : jobs, single ? J0.film_odd : nullptr);
-        mark(it, 4);
-        LMGPU_CUDA(cudaMemsetAsync(cnt + 2, 0, sizeof(int), st));
+    for (int it = 0; it < iters; it++) {
+        int *sc = it & 1 ? &c->shadow_odd : &c->shadow_even, *sc_next = it & 1 ? &c->shadow_even : &c->shadow_odd;
+        IterStamps* T = timed ? &c->it[it] : nullptr;
+        GenState G{it & 1 ? &c->started_odd : &c->started, it & 1 ? &c->started : &c->started_odd, b->job_next.as<int64_t>(),
+                   b->cap, &c->survivors[cur], &c->qn[cur], single && timed ? &T->gen : nullptr};
+        if (!single)
+            k_wf_plan<<<1, 32, 0, st>>>(ctl64(b), &c->survivors[cur], b->cap, jobs, b->job_next.as<int64_t>(), b->active.as<ActiveJob>(),
+                                        b->alloc.as<AllocEntry>(), b->first_pass, timed ? &T->gen : nullptr);
+        gen_k<<<g_gen, kBlock, 0, st>>>(jobs, b->alloc.as<AllocEntry>(), ctl64(b), G, q[cur], sq, sc);
+        ext_k<<<g_ext, kTrace, tsmem, st>>>(tb, q[cur].o, q[cur].d, &c->qn[cur], hits, &c->rays[0], &c->err, c->sums, 63, nullptr,
+                                            Fetch{&c->fetch[0], {&c->survivors[1 - cur], nullptr}, b->refill,
+                                                  timed ? T->ext : nullptr, &c->done[0]},
+                                            single ? nullptr : jobs, single ? nullptr : q[cur].job);
+        if (it > 0 && !b->image) LMGPU_CUDA(cudaStreamWaitEvent(st, shadowed, 0));
+        shade_k<<<g_shade, kBlock, 0, st>>>(jobs, q[cur], hits, &c->qn[cur], q[1 - cur], &c->survivors[1 - cur], sq, sc,
+                                            b->pass_done.as<unsigned int>(),
+                                            Resets{{&c->fetch[0], &c->fetch[1], sc_next}, timed ? &T->shade : nullptr});
+        LMGPU_CUDA(cudaEventRecord(shaded, st));
+        LMGPU_CUDA(cudaStreamWaitEvent(side, shaded, 0));
+        sh_k<<<g_sh, kTrace, tsmem, side>>>(tb, sq, sc, sfilm, &c->rays[1], &c->err, c->sums, 63, nullptr,
+                                            Fetch{&c->fetch[1], {nullptr, nullptr}, b->refill, timed ? T->shadow : nullptr, &c->done[1]},
+                                            single ? nullptr : jobs, single ? J0.film_odd : nullptr);
+        LMGPU_CUDA(cudaEventRecord(shadowed, side));
+        if (b->image || it + 1 == iters) LMGPU_CUDA(cudaStreamWaitEvent(st, shadowed, 0));
         cur = 1 - cur;
     }
     // exact count of paths in flight or not started, for the host's end-of-chunk check
-    k_wf_left<<<1, 1, 0, st>>>(ctl64(b), cnt + cur);
+    k_wf_left<<<1, 1, 0, st>>>(c, cur, timed ? 1 : 0);
 }
 
 // The executable graph for the current tuning, depth and timing; recaptured only when one of
 // them changed or a device table moved (realloc).
-cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc) {
+cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc, int iters) {
     b->refill = tuning().trace_refill;
     b->shade_minblocks = tuning().shade_minblocks;
     b->first_pass = tuning().batch_first_pass;
@@ -3483,17 +3596,28 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc) {
     const uint32_t feat = table_features(b);
     const bool same_shape = g.exec && g.depth == b->max_depth && g.refill == b->refill && g.shade == b->shade_minblocks &&
                             g.two_level == b->two_level && g.first_pass == b->first_pass && g.single == single &&
-                            g.feat == feat && g.specialize == b->specialize;
+                            g.feat == feat && g.specialize == b->specialize && g.iters == iters &&
+                            g.image == b->image;
     auto same_job = [&] {
         const JobDev& J = b->host_jobs[0];
         return std::memcmp(&g.bvh, &J.S.bvh, sizeof(Bvh8)) == 0 && g.film == J.film && g.film_odd == J.film_odd;
     };
     if (same_shape && (!single || same_job())) return g.exec;
-    if (b->timed)
-        for (auto& e : b->ev)
-            if (!e) LMGPU_CUDA(cudaEventCreate(&e));
-    cudaStream_t cs;
-    LMGPU_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
+    // the two streams and events of the capture
+    struct Capture {
+        cudaStream_t st = nullptr, side = nullptr;
+        cudaEvent_t shaded = nullptr, shadowed = nullptr;
+        ~Capture() {
+            if (shadowed) cudaEventDestroy(shadowed);
+            if (shaded) cudaEventDestroy(shaded);
+            if (side) cudaStreamDestroy(side);
+            if (st) cudaStreamDestroy(st);
+        }
+    } cap;
+    LMGPU_CUDA(cudaStreamCreateWithFlags(&cap.st, cudaStreamNonBlocking));
+    LMGPU_CUDA(cudaStreamCreateWithFlags(&cap.side, cudaStreamNonBlocking));
+    LMGPU_CUDA(cudaEventCreateWithFlags(&cap.shaded, cudaEventDisableTiming));
+    LMGPU_CUDA(cudaEventCreateWithFlags(&cap.shadowed, cudaEventDisableTiming));
     // warm-up query of grid sizes outside the capture (occupancy calls are not capturable work)
     const size_t tsmem = size_t(2) * 4 * kTrace * size_t(b->max_depth);
     (void)grid_for(b->two_level ? k_pt_extend<false, true, true> : k_pt_extend<false, true, false>, kTrace, tsmem);
@@ -3501,28 +3625,22 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc) {
     (void)grid_for(b->two_level ? k_pt_extend<false, false, true> : k_pt_extend<false, false, false>, kTrace, tsmem);
     (void)grid_for(b->two_level ? k_pt_shadow<false, false, true> : k_pt_shadow<false, false, false>, kTrace, tsmem);
     (void)grid_for(wf_shade_kernel(b, single, feat), kBlock, 0);
-    (void)grid_for(k_wf_generate, kBlock, 0);
+    (void)grid_for(k_wf_generate<true>, kBlock, 0);
+    (void)grid_for(k_wf_generate<false>, kBlock, 0);
     cudaGraph_t ng = nullptr;
     {
         // no other host thread may synchronize the device while the capture is open
         std::unique_lock<std::shared_mutex> capture_lk(capture_mutex());
-        cudaError_t began = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-        if (began != cudaSuccess) {
-            cudaStreamDestroy(cs);
-            LMGPU_CUDA(began);
-        }
+        LMGPU_CUDA(cudaStreamBeginCapture(cap.st, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_chunk(b, cs, b->timed);
+            enqueue_chunk(b, cap.st, cap.side, cap.shaded, cap.shadowed, b->timed, iters);
         } catch (...) {
             cudaGraph_t gr = nullptr;
-            cudaStreamEndCapture(cs, &gr);
+            cudaStreamEndCapture(cap.st, &gr);
             if (gr) cudaGraphDestroy(gr);
-            cudaStreamDestroy(cs);
             throw;
         }
-        cudaError_t ended = cudaStreamEndCapture(cs, &ng);
-        cudaStreamDestroy(cs);
-        LMGPU_CUDA(ended);
+        LMGPU_CUDA(cudaStreamEndCapture(cap.st, &ng));
     }
     // only the job's tree or film changed: the new graph has the same nodes, so update the
     // executable in place
@@ -3547,6 +3665,8 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc) {
     g.shade = b->shade_minblocks;
     g.specialize = b->specialize;
     g.single = single;
+    g.iters = iters;
+    g.image = b->image;
     g.feat = feat;
     if (single) {
         g.bvh = b->host_jobs[0].S.bvh;
@@ -3556,16 +3676,17 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc) {
     return g.exec;
 }
 
-// Adds one timed chunk's kernel times (events of its last launch) to b->kms: [0] extend,
-// [1] shade (with the queue-count reset before it), [2] shadow, [3] plan + generate.
-void read_chunk_times(lmgpu_batch* b) {
-    for (int it = 0; it < kChunkIters; it++) {
-        float m[4];
-        for (int k = 0; k < 4; k++) LMGPU_CUDA(cudaEventElapsedTime(&m[k], b->ev[6 * it + k], b->ev[6 * it + k + 1]));
-        b->kms[3] += m[0];
-        b->kms[0] += m[1];
-        b->kms[1] += m[2];
-        b->kms[2] += m[3];
+// Adds one timed chunk's kernel times (the stamps of its last launch) to b->kms: [0] extend, [1] shade,
+// [2] shadow (both kinds of trace launches from their start to their last block's end), [3] plan and
+// generate.
+void read_chunk_times(lmgpu_batch* b, const Ctl& h, int iters) {
+    auto ms = [](unsigned long long from, unsigned long long to) { return to > from ? double(to - from) * 1e-6 : 0.0; };
+    for (int it = 0; it < iters; it++) {
+        const IterStamps& T = h.it[it];
+        b->kms[3] += ms(T.gen, T.ext[0]);
+        b->kms[0] += ms(T.ext[0], T.ext[1]);
+        b->kms[1] += ms(T.shade, T.shadow[0]);
+        b->kms[2] += ms(T.shadow[0], T.shadow[1]);
     }
 }
 
@@ -3587,8 +3708,8 @@ int lmgpu_batch_create(lmgpu_batch** out, int64_t queue_paths) {
         }
         b->hits.alloc(c * 16);
         b->s_o.alloc(2 * c * 16); b->s_d.alloc(2 * c * 16); b->s_c.alloc(2 * c * 16); b->s_job.alloc(2 * c * 4);
-        b->ctl.alloc(256);
-        LMGPU_CUDA_SYNC(cudaMemset(b->ctl.p, 0, 256));
+        b->ctl.alloc(sizeof(Ctl));
+        LMGPU_CUDA_SYNC(cudaMemset(b->ctl.p, 0, sizeof(Ctl)));
         *out = b.release();
     });
 }
@@ -3666,6 +3787,7 @@ int lmgpu_batch_submit(lmgpu_batch* b, lmgpu_scene* s, lmgpu_film* f, const lmgp
         b->host_pass.resize(b->passes, 0);
         b->max_depth = std::max(b->max_depth, s->dev.bvh.depth);
         b->two_level = b->two_level || s->dev.num_inst > 0;
+        b->image = b->image || J.P.image;
         b->table_dirty = true;
         if (job_id) *job_id = int32_t(b->host_jobs.size() - 1);
     });
@@ -3719,34 +3841,32 @@ int lmgpu_batch_run(lmgpu_batch* b, int32_t max_chunks, void* stream, int64_t* p
             if (paths_left) *paths_left = 0;
             return;
         }
-        cudaGraphExec_t exec = ensure_graph(b, realloc);
-        cudaEvent_t e0, e1;
-        LMGPU_CUDA(cudaEventCreate(&e0));
-        LMGPU_CUDA(cudaEventCreate(&e1));
-        LMGPU_CUDA(cudaEventRecord(e0, st));
-        int64_t left = 0;
+        const int iters = chunk_iters(b, max_chunks <= 0);
+        cudaGraphExec_t exec = ensure_graph(b, realloc, iters);
+        if (!b->e0) {
+            LMGPU_CUDA(cudaEventCreate(&b->e0));
+            LMGPU_CUDA(cudaEventCreate(&b->e1));
+        }
+        LMGPU_CUDA(cudaEventRecord(b->e0, st));
+        Ctl h{};
         int chunks = 0;
-        int herr = 0;
+        const size_t words = b->timed ? sizeof(Ctl) : offsetof(Ctl, rays);
         for (;;) {
             LMGPU_CUDA(cudaGraphLaunch(exec, st));
             chunks++;
-            LMGPU_CUDA(cudaMemcpyAsync(&left, ctl64(b) + 4, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-            LMGPU_CUDA(cudaMemcpyAsync(&herr, ctl_cnt(b) + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
+            LMGPU_CUDA(cudaEventRecord(b->e1, st));
+            LMGPU_CUDA(cudaMemcpyAsync(&h, b->ctl.p, words, cudaMemcpyDeviceToHost, st));
+            LMGPU_CUDA(cudaMemcpyAsync(b->host_pass.data(), b->pass_done.p, size_t(b->passes) * 4, cudaMemcpyDeviceToHost, st));
             LMGPU_CUDA(cudaStreamSynchronize(st));
-            if (b->timed) read_chunk_times(b);
-            if (herr) throw Error(LMGPU_ERR_INTERNAL, "traversal consistency check failed");
-            if (left == 0 || (max_chunks > 0 && chunks >= max_chunks)) break;
+            if (b->timed) read_chunk_times(b, h, iters);
+            b->iters_run += iters;
+            if (h.err) throw Error(LMGPU_ERR_INTERNAL, "traversal consistency check failed");
+            if (h.left == 0 || (max_chunks > 0 && chunks >= max_chunks)) break;
         }
-        b->chunks_run += chunks;
-        LMGPU_CUDA(cudaEventRecord(e1, st));
-        LMGPU_CUDA(cudaMemcpyAsync(b->host_pass.data(), b->pass_done.p, size_t(b->passes) * 4, cudaMemcpyDeviceToHost, st));
-        LMGPU_CUDA(cudaStreamSynchronize(st));
         float ms = 0.f;
-        LMGPU_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        LMGPU_CUDA(cudaEventElapsedTime(&ms, b->e0, b->e1));
         b->elapsed_ms += ms;
-        if (paths_left) *paths_left = left;
+        if (paths_left) *paths_left = h.left;
     });
 }
 
@@ -3858,8 +3978,8 @@ int lmgpu_batch_get_stats(const lmgpu_batch* b, lmgpu_render_stats* out) {
         out->shadow_ms = b->kms[2];
         out->generate_ms = b->kms[3];
         out->trace_ms = b->kms[0] + b->kms[2];
-        out->extend_launches = b->chunks_run * kChunkIters;
-        out->shadow_launches = b->chunks_run * kChunkIters;
+        out->extend_launches = b->iters_run;
+        out->shadow_launches = b->iters_run;
     });
 }
 
@@ -3877,10 +3997,11 @@ int lmgpu_batch_reset(lmgpu_batch* b) {
         // the captured graphs stay valid: their stack depth and two-level traversal cover any
         // shallower or single-level scene, so max_depth and two_level are kept
         b->elapsed_ms = 0;
-        b->chunks_run = 0;
+        b->iters_run = 0;
         for (double& k : b->kms) k = 0;
         b->table_dirty = false;
-        LMGPU_CUDA_SYNC(cudaMemset(b->ctl.p, 0, 256));
+        LMGPU_CUDA_SYNC(cudaMemset(b->ctl.p, 0, sizeof(Ctl)));
+        b->image = false;
         if (b->pass_cap) LMGPU_CUDA_SYNC(cudaMemset(b->pass_done.p, 0, b->pass_cap * 4));
         if (b->aux_cap) LMGPU_CUDA_SYNC(cudaMemset(b->job_next.p, 0, b->aux_cap * sizeof(int64_t)));
     });
