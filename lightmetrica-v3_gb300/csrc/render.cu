@@ -824,6 +824,10 @@ __device__ inline void push_ext(const ExtQ& q, int* count, f3 o, f3 d, f3 thr, f
     store_ext<kBatched>(q, queue_slot(count), o, d, thr, pdf, n, flags, path, pixel, job);
 }
 
+// Stamps of one iteration (ns): launches' start times, and the trace launches' ends.
+struct IterStamps {
+    unsigned long long gen, ext[2], shade, shadow[2];
+};
 // Counters that a shade launch zeroes at its start (where set), for kernels that run after it and
 // that no kernel in flight uses; `stamp` receives its start time (ns).
 struct Resets {
@@ -1215,7 +1219,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_pt_shade(const __grid_co
 
 // Light paths [start, start + count): the primary ray from a sampled light (path = its index).
 __global__ void __launch_bounds__(kBlock) k_lt_generate(const __grid_constant__ DevScene S, const __grid_constant__ PtConst P,
-                                                        int64_t start, int64_t count, ExtQ q, int* qcount) {
+                                                        int64_t start, int64_t count, ExtQ q, int* qcount,
+                                                        unsigned long long* stamp) {
+    if (stamp && blockIdx.x == 0 && threadIdx.x == 0) *stamp = globaltimer_ns();
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
         const uint64_t path = uint64_t(start + i);
         float u[8];
@@ -1408,7 +1414,9 @@ __device__ inline float bd_area_pa(const DevScene& S, int light) { return (1.f /
 // its ray (sample_light_ray). Both rays go to one queue; thr.w carries the pdf_direction of the
 // ray at its origin, nrm.xyz the origin's normal.
 __global__ void __launch_bounds__(kBlock) k_bd_generate(const __grid_constant__ DevScene S, const __grid_constant__ PtConst P,
-                                                        BdRec R, int64_t start, int64_t count, ExtQ q, int* qcount) {
+                                                        BdRec R, int64_t start, int64_t count, ExtQ q, int* qcount,
+                                                        unsigned long long* stamp) {
+    if (stamp && blockIdx.x == 0 && threadIdx.x == 0) *stamp = globaltimer_ns();
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
         const uint64_t path = uint64_t(start + i);
         float u[8];
@@ -1545,7 +1553,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_bd_shade(const __grid_co
 // then the items in (t, s) order across the lanes (ballot ranks), so neighbouring items share
 // their strategy and their samples' records.
 __global__ void __launch_bounds__(kBlock) k_bd_items(BdRec R, int64_t count, int32_t min_verts, int32_t max_verts, uint2* items,
-                                                     int* icount, int64_t icap, int* err) {
+                                                     int* icount, int64_t icap, int* err, unsigned long long* stamp) {
+    if (stamp && blockIdx.x == 0 && threadIdx.x == 0) *stamp = globaltimer_ns();
     const unsigned full = 0xffffffffu;
     const int lane = int(threadIdx.x & 31u);
     const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -2062,9 +2071,12 @@ struct Workspace {
     // stream of the shadow rays that run beside the next bounce's extension rays, and the events that
     // order the two (created on first use)
     cudaStream_t side = nullptr;
-    cudaEvent_t shaded = nullptr, shadowed = nullptr;
+    cudaEvent_t shaded = nullptr, shadowed = nullptr, begun = nullptr, ended = nullptr;
+    DevBuf stamps;  // IterStamps of a timed light-traced or bidirectional render, one per bounce launched
     void ensure_side() {
         if (side) return;
+        LMGPU_CUDA(cudaEventCreate(&begun));
+        LMGPU_CUDA(cudaEventCreate(&ended));
         LMGPU_CUDA(cudaEventCreateWithFlags(&shaded, cudaEventDisableTiming));
         LMGPU_CUDA(cudaEventCreateWithFlags(&shadowed, cudaEventDisableTiming));
         LMGPU_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
@@ -2120,8 +2132,29 @@ BdConnectK bd_connect_for(uint32_t feat) {
     }
 }
 
+// Device milliseconds per kernel kind from the stamps of a render's bounces: generate up to the
+// bounce's extension launch, the trace launches to their last block's end, shade up to what follows it
+// (the next bounce's extension, the wave's connections or the shadow rays).
+struct KernelMs {
+    double gen = 0, ext = 0, shade = 0, shadow = 0;
+};
+KernelMs sum_stamps(const std::vector<IterStamps>& v) {
+    auto ms = [](unsigned long long from, unsigned long long to) { return from && to > from ? double(to - from) * 1e-6 : 0.0; };
+    KernelMs r;
+    for (size_t i = 0; i < v.size(); i++) {
+        const IterStamps& T = v[i];
+        r.gen += ms(T.gen, T.ext[0]);
+        r.ext += ms(T.ext[0], T.ext[1]);
+        const IterStamps* N = i + 1 < v.size() ? &v[i + 1] : nullptr;
+        const unsigned long long next = !N ? 0ull : N->gen ? N->gen : N->ext[0] ? N->ext[0] : N->shade;
+        r.shade += ms(T.shade, T.shadow[0] ? T.shadow[0] : next);
+        r.shadow += ms(T.shadow[0], T.shadow[1]);
+    }
+    return r;
+}
+
 void ensure_queues(Workspace& w, int64_t cap) {
-    if (!w.counters.p) w.counters.alloc(192);
+    if (!w.counters.p) w.counters.alloc(256);
     if (w.cap >= cap) return;
     for (int b = 0; b < 2; b++) {
         w.q_o[b].alloc(size_t(cap) * 16);
@@ -2698,7 +2731,7 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
             LMGPU_CUDA(cudaMemsetAsync(film, 0, size_t(npix) * 3 * 4, st));
             f->accumulated_spp = 0;
         }
-        LMGPU_CUDA(cudaMemsetAsync(ws.counters.p, 0, 192, st));
+        LMGPU_CUDA(cudaMemsetAsync(ws.counters.p, 0, 256, st));
         for (int64_t start = 0; start < total; start += wave) {
             const int64_t n = std::min(wave, total - start);
             int cur = 0;
@@ -2865,7 +2898,7 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
                         ws.q_ids[b].as<uint2>()};
         ShadowQ sq{ws.s_o.as<float4>(), ws.s_d.as<float4>(), ws.s_c.as<float4>()};
         // [0],[1] extension queues, [2],[6] shadow rays of even and odd bounces, [3] error, [4],[5] extension
-        // and shadow ray fetch
+        // and shadow ray fetch, [48],[49] finished blocks of the timed trace launches
         int* cnt = ws.counters.as<int>();
         const int refill = tuning().trace_refill;
         ws.ensure_side();
@@ -2884,39 +2917,30 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
         const int g_sh = grid_for(sh_k, kTrace, tsmem);
         const int g_shade = grid_for(shade_k, kBlock, 0);
 
-        enum { K_GEN = 0, K_EXT = 1, K_SHADE = 2, K_SHADOW = 3 };
-        std::vector<std::pair<int, cudaEvent_t>> marks;
         const bool timed = stats != nullptr;
-        auto mark = [&](int kind, cudaStream_t on = nullptr) {
-            if (!timed) return;
-            cudaEvent_t e;
-            LMGPU_CUDA(cudaEventCreate(&e));
-            LMGPU_CUDA(cudaEventRecord(e, on ? on : st));
-            marks.emplace_back(kind, e);
-        };
-        cudaEvent_t e0, e1;
-        LMGPU_CUDA(cudaEventCreate(&e0));
-        LMGPU_CUDA(cudaEventCreate(&e1));
-        int64_t n_ext = 0, n_sh = 0;
+        int64_t n_ext = 0, n_sh = 0, stamped = 0;
+        if (timed) {
+            const size_t bytes = size_t((total + wave - 1) / wave) * size_t(std::max(1, P.max_verts - 2)) * sizeof(IterStamps);
+            ws.stamps.alloc(bytes);
+            LMGPU_CUDA(cudaMemsetAsync(ws.stamps.p, 0, bytes, st));
+        }
 
-        LMGPU_CUDA(cudaEventRecord(e0, st));
+        LMGPU_CUDA(cudaEventRecord(ws.begun, st));
         if (!prm->accumulate) {
             LMGPU_CUDA(cudaMemsetAsync(film, 0, size_t(npix) * 3 * 4, st));
             f->accumulated_spp = 0;
             f->split = false;
             f->passes_even = f->passes_odd = 0;
         }
-        LMGPU_CUDA(cudaMemsetAsync(ws.counters.p, 0, 192, st));
+        LMGPU_CUDA(cudaMemsetAsync(ws.counters.p, 0, 256, st));
         // a path of max_verts <= 2 vertices cannot reach a camera connection (renderer_lt.cpp:89)
         for (int64_t start = 0; prm->max_verts > 2 && start < total; start += wave) {
             const int64_t n = std::min(wave, total - start);
             int cur = 0;
             LMGPU_CUDA(cudaMemsetAsync(cnt, 0, 12, st));
             LMGPU_CUDA(cudaMemsetAsync(cnt + 4, 0, 12, st));
-            mark(K_GEN);
             k_lt_generate<<<int(std::min<int64_t>(g_gen, (n + kBlock - 1) / kBlock)), kBlock, 0, st>>>(
-                s->dev, P, prm->first_path + start, n, q[0], cnt + 0);
-            mark(-1);
+                s->dev, P, prm->first_path + start, n, q[0], cnt + 0, timed ? &ws.stamps.as<IterStamps>()[stamped].gen : nullptr);
             LMGPU_CUDA(cudaGetLastError());
             // The ray that leaves vertex it; its hit connects when it + 1 < max_verts. A bounce's shadow
             // rays run beside the next bounce's extension rays: each launch ends with some 100 us in which
@@ -2925,24 +2949,20 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
             // counters are zeroed by launches that none of their users runs beside, not by memsets.
             for (int it = 1; it + 1 < P.max_verts; it++) {
                 int *sc = cnt + (it & 1 ? 2 : 6), *sc_next = cnt + (it & 1 ? 6 : 2);
-                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, nullptr, nullptr};
-                const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, nullptr, nullptr};
-                mark(K_EXT);
+                IterStamps* T = timed ? ws.stamps.as<IterStamps>() + stamped : nullptr;
+                stamped++;
+                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, timed ? T->ext : nullptr, cnt + 48};
+                const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, timed ? T->shadow : nullptr, cnt + 49};
                 ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
-                mark(-1);
                 n_ext++;
                 if (it > 1) LMGPU_CUDA(cudaStreamWaitEvent(st, ws.shadowed, 0));
-                mark(K_SHADE);
                 shade_k<<<g_shade, kBlock, 0, st>>>(s->dev, P, q[cur], ws.hits.as<float4>(), cnt + cur, q[1 - cur], cnt + (1 - cur),
-                                                      sq, sc, Resets{{cnt + 4, cnt + 5, sc_next}, nullptr});
-                mark(-1);
+                                                      sq, sc, Resets{{cnt + 4, cnt + 5, sc_next}, timed ? &T->shade : nullptr});
                 LMGPU_CUDA(cudaEventRecord(ws.shaded, st));
                 LMGPU_CUDA(cudaStreamWaitEvent(ws.side, ws.shaded, 0));
-                mark(K_SHADOW, ws.side);
                 sh_k<<<g_sh, kTrace, tsmem, ws.side>>>(bvh, sq, sc, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr,
                                                        nullptr);
-                mark(-1, ws.side);
                 LMGPU_CUDA(cudaEventRecord(ws.shadowed, ws.side));
                 n_sh++;
                 LMGPU_CUDA(cudaGetLastError());
@@ -2955,24 +2975,18 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
         f->scale = scale;
         k_scale<<<1024, 256, 0, st>>>(film, f->out.as<float>(), npix * 3, float(scale));
         LMGPU_CUDA(cudaGetLastError());
-        LMGPU_CUDA(cudaEventRecord(e1, st));
+        LMGPU_CUDA(cudaEventRecord(ws.ended, st));
         unsigned long long hr[2];
         int herr = 0;
+        std::vector<IterStamps> h_stamps(timed ? size_t(stamped) : 0);
+        if (!h_stamps.empty())
+            LMGPU_CUDA(cudaMemcpyAsync(h_stamps.data(), ws.stamps.p, h_stamps.size() * sizeof(IterStamps), cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaMemcpyAsync(hr, rays, sizeof(hr), cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaMemcpyAsync(&herr, cnt + 3, 4, cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaStreamSynchronize(st));
         float ms = 0.f;
-        LMGPU_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        double kms[4] = {0, 0, 0, 0};
-        for (size_t i = 0; i + 1 < marks.size(); i++) {
-            if (marks[i].first < 0) continue;
-            float m = 0.f;
-            LMGPU_CUDA(cudaEventElapsedTime(&m, marks[i].second, marks[i + 1].second));
-            kms[marks[i].first] += m;
-        }
-        for (auto& e : marks) cudaEventDestroy(e.second);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        LMGPU_CUDA(cudaEventElapsedTime(&ms, ws.begun, ws.ended));
+        const KernelMs k = sum_stamps(h_stamps);
         if (herr) throw Error(LMGPU_ERR_INTERNAL, "traversal consistency check failed");
         if (stats) {
             *stats = lmgpu_render_stats{};
@@ -2981,11 +2995,11 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
             stats->shadow_rays = int64_t(hr[1]);
             stats->rays = int64_t(hr[0] + hr[1]);
             stats->elapsed_ms = ms;
-            stats->generate_ms = kms[K_GEN];
-            stats->extend_ms = kms[K_EXT];
-            stats->shade_ms = kms[K_SHADE];
-            stats->shadow_ms = kms[K_SHADOW];
-            stats->trace_ms = kms[K_EXT] + kms[K_SHADOW];
+            stats->generate_ms = k.gen;
+            stats->extend_ms = k.ext;
+            stats->shade_ms = k.shade;
+            stats->shadow_ms = k.shadow;
+            stats->trace_ms = k.ext + k.shadow;
             stats->extend_launches = n_ext;
             stats->shadow_launches = n_sh;
         }
@@ -3051,10 +3065,10 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
             q[b] = ExtQ{ws.q_o[b].as<float4>(), ws.q_d[b].as<float4>(), ws.q_thr[b].as<float4>(), ws.q_nrm[b].as<float4>(),
                         ws.q_ids[b].as<uint2>()};
         ShadowQ sq{ws.bd_s_o.as<float4>(), ws.bd_s_d.as<float4>(), ws.bd_s_c.as<float4>()};
-        // [0],[1] extension queues, [2] connection rays, [3] error, [4],[5] ray fetch, [6] strategies
+        // [0],[1] extension queues, [2] connection rays, [3] error, [4],[5] ray fetch, [6] strategies,
+        // [48],[49] finished blocks of the timed trace launches
         int* cnt = ws.counters.as<int>();
         const int refill = tuning().trace_refill;
-        const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, nullptr, nullptr};
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
@@ -3074,59 +3088,52 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
         auto con_k = tuning().shade_minblocks <= 2 ? k_bd_connect<2> : bd_connect_for(s->dev.feat);
         const int g_con = grid_for(con_k, kBlock, 0);
 
-        enum { K_GEN = 0, K_EXT = 1, K_SHADE = 2, K_SHADOW = 3 };
-        std::vector<std::pair<int, cudaEvent_t>> marks;
         const bool timed = stats != nullptr;
-        auto mark = [&](int kind) {
-            if (!timed) return;
-            cudaEvent_t e;
-            LMGPU_CUDA(cudaEventCreate(&e));
-            LMGPU_CUDA(cudaEventRecord(e, st));
-            marks.emplace_back(kind, e);
-        };
-        cudaEvent_t e0, e1;
-        LMGPU_CUDA(cudaEventCreate(&e0));
-        LMGPU_CUDA(cudaEventCreate(&e1));
-        int64_t n_ext = 0, n_sh = 0;
+        int64_t n_ext = 0, n_sh = 0, stamped = 0;
+        ws.ensure_side();
+        if (timed) {  // per wave mv - 1 bounces, then the connections as one more
+            const size_t bytes = size_t((total + wave - 1) / wave) * size_t(mv) * sizeof(IterStamps);
+            ws.stamps.alloc(bytes);
+            LMGPU_CUDA(cudaMemsetAsync(ws.stamps.p, 0, bytes, st));
+        }
 
-        LMGPU_CUDA(cudaEventRecord(e0, st));
+        LMGPU_CUDA(cudaEventRecord(ws.begun, st));
         if (!prm->accumulate) {
             LMGPU_CUDA(cudaMemsetAsync(film, 0, size_t(npix) * 3 * 4, st));
             f->accumulated_spp = 0;
             f->split = false;
             f->passes_even = f->passes_odd = 0;
         }
-        LMGPU_CUDA(cudaMemsetAsync(ws.counters.p, 0, 192, st));
+        LMGPU_CUDA(cudaMemsetAsync(ws.counters.p, 0, 256, st));
         for (int64_t start = 0; start < total; start += wave) {
             const int64_t n = std::min(wave, total - start);
             int cur = 0;
             LMGPU_CUDA(cudaMemsetAsync(cnt, 0, 12, st));
             LMGPU_CUDA(cudaMemsetAsync(cnt + 4, 0, 8, st));
-            mark(K_GEN);
             k_bd_generate<<<int(std::min<int64_t>(g_gen, (n + kBlock - 1) / kBlock)), kBlock, 0, st>>>(
-                s->dev, P, R, prm->first_path + start, n, q[0], cnt + 0);
-            mark(-1);
+                s->dev, P, R, prm->first_path + start, n, q[0], cnt + 0, timed ? &ws.stamps.as<IterStamps>()[stamped].gen : nullptr);
             LMGPU_CUDA(cudaGetLastError());
             // the ray that leaves subpath vertex it creates vertex it + 1 (at most max_verts - 1)
             for (int it = 0; it + 1 < mv; it++) {
                 // the shade kernel zeroes the fetch counter for the next bounce's launch
-                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, nullptr, nullptr};
-                mark(K_EXT);
+                IterStamps* T = timed ? ws.stamps.as<IterStamps>() + stamped : nullptr;
+                stamped++;
+                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, timed ? T->ext : nullptr, cnt + 48};
                 ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
-                mark(-1);
                 n_ext++;
-                mark(K_SHADE);
                 shade_k<<<g_shade, kBlock, 0, st>>>(s->dev, P, R, q[cur], ws.hits.as<float4>(), cnt + cur, q[1 - cur], cnt + (1 - cur),
-                                                    Resets{{cnt + 4, nullptr, nullptr}, nullptr});
-                mark(-1);
+                                                    Resets{{cnt + 4, nullptr, nullptr}, timed ? &T->shade : nullptr});
                 LMGPU_CUDA(cudaGetLastError());
                 cur = 1 - cur;
             }
-            mark(K_SHADE);
+            // the connections' own entry: `shade` the strategy list's start, `shadow` the visibility rays
+            IterStamps* T = timed ? ws.stamps.as<IterStamps>() + stamped : nullptr;
+            stamped++;
+            const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, timed ? T->shadow : nullptr, cnt + 49};
             LMGPU_CUDA(cudaMemsetAsync(cnt + 6, 0, 4, st));
             k_bd_items<<<int(std::min<int64_t>(g_items, (n + kBlock - 1) / kBlock)), kBlock, 0, st>>>(
-                R, n, prm->min_verts, mv, ws.bd_items.as<uint2>(), cnt + 6, icap, cnt + 3);
+                R, n, prm->min_verts, mv, ws.bd_items.as<uint2>(), cnt + 6, icap, cnt + 3, timed ? &T->shade : nullptr);
             const uint2* items = ws.bd_items.as<uint2>();
             if (sort_items) {
                 int* hist = ws.bd_hist.as<int>();
@@ -3137,10 +3144,7 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
                 items = ws.bd_items_sorted.as<uint2>();
             }
             con_k<<<g_con, kBlock, 0, st>>>(s->dev, P, R, items, cnt + 6, sq, cnt + 2, scap, film, cnt + 3);
-            mark(-1);
-            mark(K_SHADOW);
             sh_k<<<g_sh, kTrace, tsmem, st>>>(bvh, sq, cnt + 2, film, rays + 1, cnt + 3, nullptr, 0, nullptr, f_sh, nullptr, nullptr);
-            mark(-1);
             n_sh++;
             LMGPU_CUDA(cudaGetLastError());
             LMGPU_CUDA(cudaMemsetAsync(cnt + 2, 0, 4, st));
@@ -3150,24 +3154,18 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
         f->scale = scale;
         k_scale<<<1024, 256, 0, st>>>(film, f->out.as<float>(), npix * 3, float(scale));
         LMGPU_CUDA(cudaGetLastError());
-        LMGPU_CUDA(cudaEventRecord(e1, st));
+        LMGPU_CUDA(cudaEventRecord(ws.ended, st));
         unsigned long long hr[2];
         int herr = 0;
+        std::vector<IterStamps> h_stamps(timed ? size_t(stamped) : 0);
+        if (!h_stamps.empty())
+            LMGPU_CUDA(cudaMemcpyAsync(h_stamps.data(), ws.stamps.p, h_stamps.size() * sizeof(IterStamps), cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaMemcpyAsync(hr, rays, sizeof(hr), cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaMemcpyAsync(&herr, cnt + 3, 4, cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaStreamSynchronize(st));
         float ms = 0.f;
-        LMGPU_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        double kms[4] = {0, 0, 0, 0};
-        for (size_t i = 0; i + 1 < marks.size(); i++) {
-            if (marks[i].first < 0) continue;
-            float m = 0.f;
-            LMGPU_CUDA(cudaEventElapsedTime(&m, marks[i].second, marks[i + 1].second));
-            kms[marks[i].first] += m;
-        }
-        for (auto& e : marks) cudaEventDestroy(e.second);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
+        LMGPU_CUDA(cudaEventElapsedTime(&ms, ws.begun, ws.ended));
+        const KernelMs k = sum_stamps(h_stamps);
         if (herr & 6) throw Error(LMGPU_ERR_INTERNAL, "connection or strategy queue overflow");
         if (herr) throw Error(LMGPU_ERR_INTERNAL, "traversal consistency check failed");
         if (stats) {
@@ -3177,11 +3175,11 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
             stats->shadow_rays = int64_t(hr[1]);
             stats->rays = int64_t(hr[0] + hr[1]);
             stats->elapsed_ms = ms;
-            stats->generate_ms = kms[K_GEN];
-            stats->extend_ms = kms[K_EXT];
-            stats->shade_ms = kms[K_SHADE];
-            stats->shadow_ms = kms[K_SHADOW];
-            stats->trace_ms = kms[K_EXT] + kms[K_SHADOW];
+            stats->generate_ms = k.gen;
+            stats->extend_ms = k.ext;
+            stats->shade_ms = k.shade;
+            stats->shadow_ms = k.shadow;
+            stats->trace_ms = k.ext + k.shadow;
             stats->extend_launches = n_ext;
             stats->shadow_launches = n_sh;
         }
@@ -3409,10 +3407,6 @@ namespace {
 constexpr int kChunkIters = 8;      // even: the queue parity is the same at every chunk boundary
 constexpr int kMaxChunkIters = 16;  // longest chunk (one job whose paths all start at once)
 
-// Stamps of one iteration (ns): launches' start times, and the trace launches' ends.
-struct IterStamps {
-    unsigned long long gen, ext[2], shade, shadow[2];
-};
 // Control words. The planner indexes the first 32 as int64 (its comment); the rest are counters, each
 // written only by launches that none of its readers runs beside.
 struct Ctl {
