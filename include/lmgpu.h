@@ -62,7 +62,8 @@ int lmgpu_version(void);
  *                   rays once fewer than this many lanes still trace (1..32; default 24); 0 runs
  *                   one ray per thread without refills.
  *   "shade_minblocks" shade kernels: 256-thread blocks per SM their register budget must allow
- *                   (2: up to 128 registers; 3: up to 80; 4: up to 64, the default).
+ *                   (2: up to 128 registers; 3: up to 80; 4: up to 64, the default, at which
+ *                   kernels specialised for a scene's features use their own measured choice).
  *   "batch_first_pass" shared wavefront: start the sample-0 paths of every job before any other
  *                   path (1, the default: a newly admitted job's first image does not wait behind
  *                   older jobs' later samples) or start paths in submission order (0).

@@ -682,7 +682,9 @@ __device__ inline void splat(float* film, uint32_t pixel, f3 c) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Wavefront state
+// Wavefront state. Queue entries are written once and read once or twice per bounce, gigabytes of them
+// in a large render; the streaming (evict-first) accesses keep them from pushing nodes and shading
+// records out of L2 (1080p frame at 16 spp: shade 7.45 -> 7.21 ms, 28.7 -> 28.3 ms in all).
 struct ExtQ {
     float4* o;     // origin (w unused)
     float4* d;     // direction (w unused)
@@ -753,10 +755,10 @@ __device__ inline int queue_slot(int* count) {
 template <bool kBatched>
 __device__ inline void push_shadow(const ShadowQ& sq, int* count, f3 o, f3 d, float tmax, f3 c, uint32_t pixel, uint32_t job) {
     const int k = queue_slot(count);
-    sq.o[k] = make_float4(o.x, o.y, o.z, tmax);
-    sq.d[k] = make_float4(d.x, d.y, d.z, 0.f);
-    sq.c[k] = make_float4(c.x, c.y, c.z, __uint_as_float(pixel));
-    if (kBatched) sq.job[k] = job;
+    __stcs(sq.o + k, make_float4(o.x, o.y, o.z, tmax));
+    __stcs(sq.d + k, make_float4(d.x, d.y, d.z, 0.f));
+    __stcs(sq.c + k, make_float4(c.x, c.y, c.z, __uint_as_float(pixel)));
+    if (kBatched) __stcs(sq.job + k, job);
 }
 
 __device__ inline uint32_t pixel_of(const PtConst& P, float rx, float ry) {
@@ -811,12 +813,12 @@ __device__ inline void nee(const DevScene& S, const PtConst& P, const Geom& g, c
 template <bool kBatched>
 __device__ inline void store_ext(const ExtQ& q, int64_t k, f3 o, f3 d, f3 thr, float pdf, f3 n, uint32_t flags, uint32_t path,
                                  uint32_t pixel, uint32_t job) {
-    q.o[k] = make_float4(o.x, o.y, o.z, 0.f);
-    q.d[k] = make_float4(d.x, d.y, d.z, 0.f);
-    q.thr[k] = make_float4(thr.x, thr.y, thr.z, pdf);
-    q.nrm[k] = make_float4(n.x, n.y, n.z, __uint_as_float(flags));
-    q.ids[k] = make_uint2(path, pixel);
-    if (kBatched) q.job[k] = job;
+    __stcs(q.o + k, make_float4(o.x, o.y, o.z, 0.f));
+    __stcs(q.d + k, make_float4(d.x, d.y, d.z, 0.f));
+    __stcs(q.thr + k, make_float4(thr.x, thr.y, thr.z, pdf));
+    __stcs(q.nrm + k, make_float4(n.x, n.y, n.z, __uint_as_float(flags)));
+    __stcs(q.ids + k, make_uint2(path, pixel));
+    if (kBatched) __stcs(q.job + k, job);
 }
 template <bool kBatched>
 __device__ inline void push_ext(const ExtQ& q, int* count, f3 o, f3 d, f3 thr, float pdf, f3 n, uint32_t flags, uint32_t path,
@@ -986,12 +988,12 @@ __global__ void __launch_bounds__(kTrace, kExtendBlocks) k_pt_extend(Bvh8 bvh, c
         fetch_loop<false, kCount, kTwoLevel>(
             n, int(gridDim.x * (blockDim.x / 32)), f, stk, int(blockDim.x), &lerr,
             [&](int k, Trav& s) {
-                const float4 o = qo[k], d = qd[k];
+                const float4 o = __ldcs(qo + k), d = __ldcs(qd + k);
                 trav_init(s, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, kInf);
             },
             [&](int k) -> Bvh8 { return kBatched ? jobs[qjob[k]].S.bvh : bvh; },
             [&](int k, const Trav& s) {
-                hits[k] = make_float4(s.best.t, s.best.u, s.best.v, __int_as_float(s.best.id));
+                __stcs(hits + k, make_float4(s.best.t, s.best.u, s.best.v, __int_as_float(s.best.id)));
                 if (kCount && (k & count_mask) == 0) {
                     cn += s.nvis;
                     ct += s.ntri;
@@ -1002,7 +1004,7 @@ __global__ void __launch_bounds__(kTrace, kExtendBlocks) k_pt_extend(Bvh8 bvh, c
             });
     } else {
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-            const float4 o = qo[k], d = qd[k];
+            const float4 o = __ldcs(qo + k), d = __ldcs(qd + k);
             const Bvh8& B = kBatched ? jobs[qjob[k]].S.bvh : bvh;
             TraceHit h;
             if (kCount && (k & count_mask) == 0) {
@@ -1050,7 +1052,7 @@ __global__ void __launch_bounds__(kTrace, kShadowBlocks) k_pt_shadow(Bvh8 bvh, S
         fetch_loop<true, kCount, kTwoLevel>(
             n, int(gridDim.x * (blockDim.x / 32)), f, stk, int(blockDim.x), &lerr,
             [&](int k, Trav& s) {
-                const float4 o = sq.o[k], d = sq.d[k];
+                const float4 o = __ldcs(sq.o + k), d = __ldcs(sq.d + k);
                 trav_init(s, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), kEps, o.w);
             },
             [&](int k) -> Bvh8 { return kBatched ? jobs[sq.job[k]].S.bvh : bvh; },
@@ -1070,7 +1072,7 @@ __global__ void __launch_bounds__(kTrace, kShadowBlocks) k_pt_shadow(Bvh8 bvh, S
             });
     } else {
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-            const float4 o = sq.o[k], d = sq.d[k];
+            const float4 o = __ldcs(sq.o + k), d = __ldcs(sq.d + k);
             const uint32_t job = kBatched ? sq.job[k] : 0u;
             const Bvh8& B = kBatched ? jobs[job].S.bvh : bvh;
             TraceHit h;
@@ -1859,11 +1861,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_wf_shade(const JobDev* _
     reset_counters(resets);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         // kSingle: the batch holds one job, so no per-path job id is read
-        const uint32_t job = kSingle ? 0u : qi.job[k];
+        const uint32_t job = kSingle ? 0u : __ldcs(qi.job + k);
         const JobDev& J = jobs[job];
-        const uint2 ids = qi.ids[k];
-        const bool alive = shade_path<true, kF>(J.S, J.P, J.film, J.film_odd, J.parity0, job, qi.o[k], qi.d[k], qi.thr[k], qi.nrm[k], hits[k], ids, qo,
-                                            qocount, sq, scount);
+        const uint2 ids = __ldcs(qi.ids + k);
+        const bool alive = shade_path<true, kF>(J.S, J.P, J.film, J.film_odd, J.parity0, job, __ldcs(qi.o + k), __ldcs(qi.d + k),
+                                                   __ldcs(qi.thr + k), __ldcs(qi.nrm + k), __ldcs(hits + k), ids, qo, qocount, sq, scount);
         if (!alive) {
             const uint32_t key = J.pass_off + ids.x % uint32_t(J.P.spp);
             // the lanes that end paths of one pass share one atomic (sample-major order puts them
@@ -3458,13 +3460,13 @@ __global__ void k_wf_set_total(int64_t* ctl, int64_t total, int64_t njobs) {
     ctl[5] = njobs;
 }
 
-// The one-job shade kernel specialised for the job scene's features (default register budget).
-#ifndef LMGPU_SHADE_SINGLE_MINBLOCKS
-#define LMGPU_SHADE_SINGLE_MINBLOCKS 4  // blocks per SM of the specialised kernels (3: 41.0 ms, 5: 39.5 ms, 4: 37.1 ms per frame)
-#endif
+// The one-job shade kernel specialised for the job scene's features, at two 256-thread blocks per SM
+// (up to 128 registers, no spills). The 1080p frame at 16 spp: 4 blocks (64 registers) 8.35 ms of
+// shade, 3: 7.85, 2: 7.2-7.6; 16.6M paths of a 540k-triangle scene 2.66, 2.56, 2.26. Kernels of a job
+// table keep four: 16 batched jobs 16.05 ms, 16.1 at three, 16.6 at two.
 using WfShadeK = decltype(&k_wf_shade<4, true, kFeatAll>);
 WfShadeK wf_shade_single(uint32_t feat) {
-    constexpr int mb = LMGPU_SHADE_SINGLE_MINBLOCKS;
+    constexpr int mb = 2;
     if (feat & (kFeatDelta | kFeatTexture)) return k_wf_shade<mb, true, kFeatAll>;
     switch (feat & 7u) {
     case 0: return k_wf_shade<mb, true, 0u>;
