@@ -62,6 +62,13 @@ __device__ inline float refine_hit_t(const float4 ra, const float4 rb, const flo
     return lmgpu_ht::hit_t(o, d, p1, e1, e2);
 }
 
+__device__ inline void refine_hit(const float4* rays, lmgpu_hit* hits, int64_t i, const float4* tris, const int32_t* tri_slot) {
+    const int32_t id = hits[i].prim;
+    if (id < 0) return;
+    const float4* tp = tris + size_t(__ldg(tri_slot + id)) * 3;
+    hits[i].t = refine_hit_t(rays[2 * i], rays[2 * i + 1], __ldg(tp), __ldg(tp + 1), __ldg(tp + 2));
+}
+
 // rays: 2 float4 per ray (o, tmin) (d, tmax). refill > 0: block b of G takes the groups of
 // 2^group_log2 consecutive rays b, b + G, b + 2G, ... and its warps fetch from them dynamically through a
 // shared-memory counter (no state outside the launch, so calls on several streams may overlap).
@@ -69,10 +76,11 @@ __device__ inline float refine_hit_t(const float4 ra, const float4 rb, const flo
 // chunk per block, rays in caller order (camera rays, bounces sorted by origin or direction) left
 // some blocks all the expensive rays, and a batch of diffuse bounces in pixel order traced 11 %
 // slower than the same rays shuffled. refill == 0: one ray per thread, grid-stride.
-template <bool kAnyHit, bool kTwoLevel>
+// kRefine (closest hits, single level, refill > 0): the block also refines its own hits' distances.
+template <bool kAnyHit, bool kTwoLevel, bool kRefine = false>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(Bvh8 bvh, const float4* __restrict__ rays, int64_t n,
                                                             lmgpu_hit* __restrict__ hits, uint8_t* __restrict__ occluded,
-                                                            int* __restrict__ err, int refill, int group_log2) {
+                                                            int* __restrict__ err, int refill, int group_log2, const int32_t* __restrict__ tri_slot) {
     extern __shared__ uint2 smem[];
     __shared__ int s_fetch;
     const int stride = blockDim.x;
@@ -108,6 +116,11 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(Bvh8 bvh, const flo
                 trav_init(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w);
             },
             [&](int) { return bvh; }, [&](int k, const Trav& s) { store(ray_of(k), s.best); });
+        if (kRefine) {
+            __syncthreads();  // the block's hits are written
+            for (int k = threadIdx.x; k < int(count); k += blockDim.x)
+                refine_hit(rays, hits, ray_of(k), bvh.tris, tri_slot);
+        }
     } else {
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
             const float4 a = rays[2 * i], b = rays[2 * i + 1];
@@ -118,18 +131,14 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(Bvh8 bvh, const flo
     if (lerr) atomicOr(err, lerr);
 }
 
-// The fp64 hit distance of every closest hit (refine_hit_t), as a pass of its own after the
-// trace: inside the persistent traversal loop the lanes whose ray ends would run its long chain
-// of double ops while the warp's other lanes wait.
+// The fp64 hit distance of every closest hit, as a pass of its own after the trace: inside the
+// persistent traversal loop the lanes whose ray ends would run its long chain while the warp's other
+// lanes wait (2^24-ray probe 3632 -> 4440 us, with the lanes that end together at a refill).
 __global__ void __launch_bounds__(256) k_refine_hits(const float4* __restrict__ rays, lmgpu_hit* __restrict__ hits,
                                                      int64_t n, const float4* __restrict__ tris,
                                                      const int32_t* __restrict__ tri_slot) {
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        const int32_t id = hits[i].prim;
-        if (id < 0) continue;
-        const float4* tp = tris + size_t(__ldg(tri_slot + id)) * 3;
-        hits[i].t = refine_hit_t(rays[2 * i], rays[2 * i + 1], __ldg(tp), __ldg(tp + 1), __ldg(tp + 2));
-    }
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
+        refine_hit(rays, hits, i, tris, tri_slot);
 }
 
 // Instrumented pass: node visits and triangle tests summed over every `sample`-th ray.
@@ -188,6 +197,11 @@ void launch_trace(const lmgpu_accel* a, const void* d_rays, int64_t n, void* d_h
         throw Error(LMGPU_ERR_INVALID_ARGUMENT, "ray buffer must be 16-byte aligned");
     const Bvh8 b = device_view(a);
     const size_t smem = trace_smem(a);
+    const bool two = a->num_instances > 0, refine = !d_occ && !two && a->tri_slot.p;
+    // Batches of at most one ray per resident lane refine their hits in the trace launch: 2^10 rays
+    // 66.7 -> 60.7 us, 2^17 178 -> 174. Larger ones in a launch of their own: with the refinement's
+    // code the trace kernel takes 79 instead of 72 registers (2^20 rays 616 -> 644 us).
+    const bool fused = refine && tuning().trace_refill > 0 && n <= int64_t(current_device().num_sms) * 1024;
     auto run = [&](auto kernel) {
         // Rays per group: 32, or fewer when the batch has fewer rays than the chip has lanes, so that
         // they spread over all warps; down to the four rays of a cooperative warp.
@@ -197,13 +211,14 @@ void launch_trace(const lmgpu_accel* a, const void* d_rays, int64_t n, void* d_h
         const int64_t groups = (n + (int64_t(1) << gl) - 1) >> gl;
         const int g = int(std::min<int64_t>(gmax, tuning().trace_refill > 0 ? (groups + warps - 1) / warps : (n + kTraceBlock - 1) / kTraceBlock));
         kernel<<<g, kTraceBlock, smem, st>>>(b, static_cast<const float4*>(d_rays), n, static_cast<lmgpu_hit*>(d_hits), d_occ,
-                                             d_err, tuning().trace_refill, gl);
+                                             d_err, tuning().trace_refill, gl, a->tri_slot.as<const int32_t>());
     };
-    const bool two = a->num_instances > 0;
     if (d_occ) two ? run(k_trace_batch<true, true>) : run(k_trace_batch<true, false>);
-    else two ? run(k_trace_batch<false, true>) : run(k_trace_batch<false, false>);
+    else if (two) run(k_trace_batch<false, true>);
+    else if (fused) run(k_trace_batch<false, false, true>);
+    else run(k_trace_batch<false, false>);
     LMGPU_CUDA(cudaGetLastError());
-    if (!d_occ && !two && a->tri_slot.p && n > 0) {
+    if (refine && !fused) {
         const int g = int(std::min<int64_t>((n + 255) / 256, int64_t(current_device().num_sms) * 8));
         k_refine_hits<<<g, 256, 0, st>>>(static_cast<const float4*>(d_rays), static_cast<lmgpu_hit*>(d_hits), n,
                                          a->tris.as<const float4>(), a->tri_slot.as<const int32_t>());
