@@ -1198,6 +1198,59 @@ __device__ __forceinline__ bool shade_path(const DevScene& S, const PtConst& P, 
     return true;
 }
 
+// The block's entries [base, base + kBlock) of the queue in order of what their rays met -- nothing, then
+// by material type -- so that warps of a later bounce run one kind of shading instead of all of them
+// (8.5 of 32 lanes were active there): the calling thread's place in that order, as an offset from
+// `base`; entries past `n` come last. The record's line and the tables are read again by the shading
+// itself, from L1. 1080p frame at 16 spp 27.9 -> 26.5 ms, sixteen batched jobs 15.6 -> 14.8, frame of
+// 2^22 light paths 4.07 -> 3.97; bidirectional shading, whose lanes do less per vertex, lost 2 % and
+// keeps the queue's order. Two-level trees order by hit and miss only. Called by all threads of the
+// block; `turn` alternates between calls (two barriers a call: a call's buffers are next written two
+// calls later).
+constexpr int kShadeKinds = 8;
+template <uint32_t kF, typename SceneOf>
+__device__ __forceinline__ int shade_order(const float4* __restrict__ hits, int base, int n, int turn, SceneOf scene_of) {
+    constexpr int kWarps = kBlock / 32;
+    static_assert(kShadeKinds * kWarps == 64, "two counters per lane");
+    __shared__ int counts[2][kShadeKinds * kWarps];
+    __shared__ unsigned char order[2][kBlock];
+    const int k = base + int(threadIdx.x), lane = int(threadIdx.x & 31u), warp = int(threadIdx.x >> 5);
+    int kind = kShadeKinds - 1;
+    if (k < n) {
+        const int32_t id = __float_as_int(__ldcs(hits + k).w);
+        kind = id < 0 ? 0 : 1;
+        if (id >= 0 && !(kF & kFeatTwoLevel)) {
+            const DevScene& S = scene_of(k);
+            const int32_t prim = __float_as_int(__ldg(S.shade + size_t(id) * 6 + 5).y);
+            kind = 1 + S.mats[__ldg(S.prim_ml + prim).x].type;
+        }
+    }
+    int rank = 0;
+#pragma unroll
+    for (int q = 0; q < kShadeKinds; q++) {
+        const unsigned m = __ballot_sync(0xffffffffu, kind == q);
+        if (kind == q) rank = __popc(m & ((1u << lane) - 1u));
+        if (lane == q) counts[turn][q * kWarps + warp] = __popc(m);
+    }
+    __syncthreads();
+    // exclusive prefix sums of the 64 counters, by every warp for itself
+    const int c0 = counts[turn][lane], c1 = counts[turn][lane + 32];
+    int s0 = c0, s1 = c1;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u0 = __shfl_up_sync(0xffffffffu, s0, o), u1 = __shfl_up_sync(0xffffffffu, s1, o);
+        if (lane >= o) {
+            s0 += u0;
+            s1 += u1;
+        }
+    }
+    s1 += __shfl_sync(0xffffffffu, s0, 31);
+    const int at = kind * kWarps + warp;
+    const int b0 = __shfl_sync(0xffffffffu, s0 - c0, at & 31), b1 = __shfl_sync(0xffffffffu, s1 - c1, at & 31);
+    order[turn][(at < 32 ? b0 : b1) + rank] = static_cast<unsigned char>(threadIdx.x);
+    __syncthreads();
+    return order[turn][threadIdx.x];
+}
+
 // kMinBlocks: resident 256-thread blocks per SM the register allocation must allow (2: up to 128
 // registers; 3: 80; 4: 64), selected at run time by the "shade_minblocks" tuning key.
 template <int kMinBlocks>
@@ -1244,7 +1297,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_lt_shade(const __grid_co
                                                      ExtQ qo, int* qocount, ShadowQ sq, int* scount, Resets resets) {
     const int n = *qicount;
     reset_counters(resets);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    for (int first = blockIdx.x * kBlock, turn = 0; first < n; first += gridDim.x * kBlock, turn ^= 1) {
+        const int k = first + shade_order<kF>(hits, first, n, turn, [&](int) -> const DevScene& { return S; });
+        if (k >= n) continue;
         const float4 h4 = hits[k];
         const int32_t id = __float_as_int(h4.w);
         if (id < 0) continue;  // no surface (or the environment): the walk ends
@@ -1859,7 +1914,9 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_wf_shade(const JobDev* _
                                                      int* scount, unsigned int* pass_done, Resets resets) {
     const int n = *qicount;
     reset_counters(resets);
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    for (int first = blockIdx.x * kBlock, turn = 0; first < n; first += gridDim.x * kBlock, turn ^= 1) {
+        const int k = first + shade_order<kF>(hits, first, n, turn, [&](int i) -> const DevScene& { return jobs[kSingle ? 0u : __ldcs(qi.job + i)].S; });
+        if (k >= n) continue;
         // kSingle: the batch holds one job, so no per-path job id is read
         const uint32_t job = kSingle ? 0u : __ldcs(qi.job + k);
         const JobDev& J = jobs[job];
@@ -2098,15 +2155,15 @@ Workspace& workspace(int device) {
 
 // Light-tracing and BDPT kernels specialised on the features they use: instances and mixture
 // materials (shade), the textured environment and mixture materials (connect).
-// Three resident blocks per SM (up to 80 registers) rather than four (64 registers, up to 48
-// bytes of stack): the LT frame 16.04 -> 15.72 ms (A/B on one GB300, three alternating runs each).
-using LtShadeK = decltype(&k_lt_shade<3, kFeatAll>);
+// Four resident blocks per SM: with the entries in order of material, the frame of 2^22 light paths
+// takes 3.97 ms, 4.04 at three blocks and 4.24 at two.
+using LtShadeK = decltype(&k_lt_shade<4, kFeatAll>);
 LtShadeK lt_shade_for(uint32_t feat) {
     switch (feat & (kFeatMixture | kFeatTwoLevel)) {
-    case 0: return k_lt_shade<3, 0u>;
-    case kFeatMixture: return k_lt_shade<3, kFeatMixture>;
-    case kFeatTwoLevel: return k_lt_shade<3, kFeatTwoLevel>;
-    default: return k_lt_shade<3, kFeatMixture | kFeatTwoLevel>;
+    case 0: return k_lt_shade<4, 0u>;
+    case kFeatMixture: return k_lt_shade<4, kFeatMixture>;
+    case kFeatTwoLevel: return k_lt_shade<4, kFeatTwoLevel>;
+    default: return k_lt_shade<4, kFeatMixture | kFeatTwoLevel>;
     }
 }
 // Three resident blocks per SM (up to 80 registers, no spills) rather than four (64 registers,
@@ -3460,13 +3517,13 @@ __global__ void k_wf_set_total(int64_t* ctl, int64_t total, int64_t njobs) {
     ctl[5] = njobs;
 }
 
-// The one-job shade kernel specialised for the job scene's features, at two 256-thread blocks per SM
-// (up to 128 registers, no spills). The 1080p frame at 16 spp: 4 blocks (64 registers) 8.35 ms of
-// shade, 3: 7.85, 2: 7.2-7.6; 16.6M paths of a 540k-triangle scene 2.66, 2.56, 2.26. Kernels of a job
-// table keep four: 16 batched jobs 16.05 ms, 16.1 at three, 16.6 at two.
+// The one-job shade kernel specialised for the job scene's features, at three 256-thread blocks per SM:
+// 1080p frame at 16 spp 26.5 ms (2 blocks 26.5, 4 blocks 26.9), 16.6M paths of a 540k-triangle scene
+// 9.28 (9.86, 9.73), 64 instances 5.35 (5.52, 5.30). Kernels of a job table keep four: sixteen batched
+// jobs 14.8 ms, 15.05 at three, 15.8 at two.
 using WfShadeK = decltype(&k_wf_shade<4, true, kFeatAll>);
 WfShadeK wf_shade_single(uint32_t feat) {
-    constexpr int mb = 2;
+    constexpr int mb = 3;
     if (feat & (kFeatDelta | kFeatTexture)) return k_wf_shade<mb, true, kFeatAll>;
     switch (feat & 7u) {
     case 0: return k_wf_shade<mb, true, 0u>;
