@@ -384,7 +384,8 @@ def run_gpu(args) -> None:
 
     # kernels per step: every chunk of the shared wavefront launches extend, shade, shadow, plan and
     # generate once per bounce iteration; one film resolve per render
-    launches_per_step = 5 * tot["ext_launches"] / max(1, args.steps) + 1
+    # per iteration generate, extend, shade and shadow; the film scaling
+    launches_per_step = 4 * tot["ext_launches"] / max(1, args.steps) + 1
     if rank == 0:
         out = {
             "metric": METRIC, "value": value, "unit": "Mrays/s", "n_gpus": ws, "steps": args.steps,

@@ -3435,6 +3435,7 @@ struct lmgpu_batch {
         bool single = false;      // captured for a one-job table
         uint32_t feat = 0;        // that job's scene features (the shade kernel specialised for them)
         lmgpu::Bvh8 bvh{};        // that job's tree and films, passed by value to the trace kernels
+        std::vector<cudaGraphNode_t> ext_nodes, sh_nodes;  // whose launches hold them
         float* film = nullptr;
         float* film_odd = nullptr;
         void clear() {
@@ -3442,6 +3443,8 @@ struct lmgpu_batch {
             if (graph) cudaGraphDestroy(graph);
             exec = nullptr;
             graph = nullptr;
+            ext_nodes.clear();
+            sh_nodes.clear();
         }
     } slot[2];
     int refill = 0, shade_minblocks = 3, first_pass = 1, specialize = 1;
@@ -3561,7 +3564,17 @@ int chunk_iters(const lmgpu_batch* b, bool to_end) {
 
 // Stream-ordered view of one chunk of iterations; captured into a graph. `side`: a second stream of
 // the capture, with events `shaded` and `shadowed` between the two.
-void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent_t shaded, cudaEvent_t shadowed, bool timed, int iters) {
+void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent_t shaded, cudaEvent_t shadowed, bool timed, int iters,
+                   std::vector<cudaGraphNode_t>& ext_nodes, std::vector<cudaGraphNode_t>& sh_nodes) {
+    // the node of the launch last captured on a stream
+    auto node_of = [](cudaStream_t on) {
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t* deps = nullptr;
+        size_t n = 0;
+        LMGPU_CUDA(cudaStreamGetCaptureInfo(on, &status, nullptr, nullptr, &deps, nullptr, &n));
+        if (status != cudaStreamCaptureStatusActive || n != 1) throw Error(LMGPU_ERR_INTERNAL, "stream capture lost a launch");
+        return deps[0];
+    };
     const size_t tsmem = size_t(2) * 4 * kTrace * size_t(b->max_depth);
     Bvh8 bmax{};
     bmax.depth = b->max_depth;
@@ -3616,6 +3629,8 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent
                                             Fetch{&c->fetch[0], {&c->survivors[1 - cur], nullptr}, b->refill,
                                                   timed ? T->ext : nullptr, &c->done[0]},
                                             single ? nullptr : jobs, single ? nullptr : q[cur].job);
+        LMGPU_CUDA(cudaGetLastError());
+        ext_nodes.push_back(node_of(st));
         if (it > 0 && !b->image) LMGPU_CUDA(cudaStreamWaitEvent(st, shadowed, 0));
         shade_k<<<g_shade, kBlock, 0, st>>>(jobs, q[cur], hits, &c->qn[cur], q[1 - cur], &c->survivors[1 - cur], sq, sc,
                                             b->pass_done.as<unsigned int>(),
@@ -3625,6 +3640,8 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent
         sh_k<<<g_sh, kTrace, tsmem, side>>>(tb, sq, sc, sfilm, &c->rays[1], &c->err, c->sums, 63, nullptr,
                                             Fetch{&c->fetch[1], {nullptr, nullptr}, b->refill, timed ? T->shadow : nullptr, &c->done[1]},
                                             single ? nullptr : jobs, single ? J0.film_odd : nullptr);
+        LMGPU_CUDA(cudaGetLastError());
+        sh_nodes.push_back(node_of(side));
         LMGPU_CUDA(cudaEventRecord(shadowed, side));
         if (b->image || it + 1 == iters) LMGPU_CUDA(cudaStreamWaitEvent(st, shadowed, 0));
         cur = 1 - cur;
@@ -3656,6 +3673,28 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc, int iters) {
         return std::memcmp(&g.bvh, &J.S.bvh, sizeof(Bvh8)) == 0 && g.film == J.film && g.film_odd == J.film_odd;
     };
     if (same_shape && (!single || same_job())) return g.exec;
+    if (same_shape) {
+        // only the job's tree or films changed: new arguments for the trace launches (16 of 33 nodes; a new
+        // capture and cudaGraphExecUpdate took 60 us of a 350 us preview, this 9)
+        const JobDev& J = b->host_jobs[0];
+        Bvh8 tb = J.S.bvh;
+        tb.depth = b->max_depth;
+        float *film = J.film, *film_odd = J.film_odd;
+        auto set = [&](cudaGraphNode_t node, std::initializer_list<std::pair<int, void*>> changed, int count) {
+            cudaKernelNodeParams kp{};
+            LMGPU_CUDA(cudaGraphKernelNodeGetParams(node, &kp));
+            std::vector<void*> args(kp.kernelParams, kp.kernelParams + count);
+            for (const auto& c : changed) args[size_t(c.first)] = c.second;
+            kp.kernelParams = args.data();
+            LMGPU_CUDA(cudaGraphExecKernelNodeSetParams(g.exec, node, &kp));
+        };
+        for (auto node : g.ext_nodes) set(node, {{0, &tb}}, 13);
+        for (auto node : g.sh_nodes) set(node, {{0, &tb}, {3, &film}, {11, &film_odd}}, 12);
+        g.bvh = J.S.bvh;
+        g.film = film;
+        g.film_odd = film_odd;
+        return g.exec;
+    }
     // the two streams and events of the capture
     struct Capture {
         cudaStream_t st = nullptr, side = nullptr;
@@ -3681,12 +3720,13 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc, int iters) {
     (void)grid_for(k_wf_generate<true>, kBlock, 0);
     (void)grid_for(k_wf_generate<false>, kBlock, 0);
     cudaGraph_t ng = nullptr;
+    std::vector<cudaGraphNode_t> ext_nodes, sh_nodes;
     {
         // no other host thread may synchronize the device while the capture is open
         std::unique_lock<std::shared_mutex> capture_lk(capture_mutex());
         LMGPU_CUDA(cudaStreamBeginCapture(cap.st, cudaStreamCaptureModeThreadLocal));
         try {
-            enqueue_chunk(b, cap.st, cap.side, cap.shaded, cap.shadowed, b->timed, iters);
+            enqueue_chunk(b, cap.st, cap.side, cap.shaded, cap.shadowed, b->timed, iters, ext_nodes, sh_nodes);
         } catch (...) {
             cudaGraph_t gr = nullptr;
             cudaStreamEndCapture(cap.st, &gr);
@@ -3695,22 +3735,11 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc, int iters) {
         }
         LMGPU_CUDA(cudaStreamEndCapture(cap.st, &ng));
     }
-    // only the job's tree or film changed: the new graph has the same nodes, so update the
-    // executable in place
-    bool updated = false;
-    if (same_shape) {
-        cudaGraphExecUpdateResultInfo info;
-        updated = cudaGraphExecUpdate(g.exec, ng, &info) == cudaSuccess;
-        if (!updated) (void)cudaGetLastError();
-    }
-    if (updated) {
-        if (g.graph) cudaGraphDestroy(g.graph);
-        g.graph = ng;
-    } else {
-        g.clear();
-        g.graph = ng;
-        LMGPU_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
-    }
+    g.clear();
+    g.graph = ng;
+    LMGPU_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
+    g.ext_nodes = std::move(ext_nodes);
+    g.sh_nodes = std::move(sh_nodes);
     g.depth = b->max_depth;
     g.refill = b->refill;
     g.two_level = b->two_level;
