@@ -1,5 +1,5 @@
-// Accel C-ABI (include/lmgpu.h): build the 8-wide BVH on the host, keep it resident on the
-// device, and trace batches of rays with one thread per ray.
+// Accel C-ABI (include/lmgpu.h): build the 8-wide BVH on the host or the GPU, keep it resident on the
+// device, and trace batches of rays with persistent warps that fetch them dynamically.
 #include <algorithm>
 #include <array>
 #include <cmath>
