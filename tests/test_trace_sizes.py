@@ -76,3 +76,20 @@ def test_batch_sizes(lm, native_lib, oracle_mod, two_level):
         ok[[7, 11, 13]] = False
         t, uv, ids, _ = S.intersect(rays[ok], brute=True, refine_t=True)
         compare_bitexact(big[ok], t, uv, ids, rays[ok], S.triangles())
+
+
+@pytest.mark.parametrize("far", [0.0, 0.5, 0.97, 1.0])  # rays from far away: all but a few miss
+@pytest.mark.parametrize("n", [32 * WARP_ROOM + 1, 64 * WARP_ROOM + 31, 500001])
+def test_distance_pass(lm, n, far):
+    """Larger batches take the hit distances in a pass of its own, whose warps collect the hits of the
+    rays they pass: the bits of the same rays in batches whose trace launch takes them."""
+    accel = lm.load_accel("accel", "sahbvh")
+    accel.build_triangles(_soup(700, 5))
+    rays = _rays(n, 17)
+    rays[:, :3] = 0.5
+    rays[np.random.default_rng(3).random(n) < far, :3] = 50.0
+    rays[:, 7] = 1e10
+    out = accel.intersect_batch(rays)
+    step = 100003
+    parts = b"".join(accel.intersect_batch(rays[i:i + step]).tobytes() for i in range(0, n, step))
+    assert out.tobytes() == parts
