@@ -201,7 +201,10 @@ __device__ inline void trav_set_ray(Trav& s, f3 o, f3 d) {
 
 __device__ inline void trav_init(Trav& s, f3 o, f3 d, float tmin, float tmax) {
     trav_set_ray(s, o, d);
-    s.tmin = tmin;
+    // -0 for a zero: the box comparison is the sign of far * kWiden - near, and a hit at t = -0 (a ray
+    // that starts on a surface) as the far side against +0 gives -0, a miss of boxes with hits at the
+    // same t and a smaller index; against -0 it gives +0.
+    s.tmin = tmin == 0.0f ? -0.0f : tmin;
     s.best = TraceHit{tmax, 0.f, 0.f, -1};
     s.sp = 0;
     s.node = 0;
@@ -246,7 +249,8 @@ __device__ __forceinline__ uint32_t node_children(const uint4& w0, const uint4& 
     const uint32_t nz0 = oz ? w4.z : w3.x, nz1 = oz ? w4.w : w3.y, fz0 = oz ? w3.x : w4.z, fz1 = oz ? w3.y : w4.w;
     // The trace kernels are bound by instruction issue (70-79 % of the slots, the nodes in L1 and L2),
     // a node's 48 planes being most of it: two slots per instruction (fma.f32x2), and the comparison
-    // near <= far * kWiden as the sign of far * kWiden - near shifted into the mask, slot 7 first
+    // near <= far * kWiden as the sign of far * kWiden - near shifted into the mask, slot 7 first (zeros:
+    // see trav_init)
     // (2^20 diffuse bounces in a soup of 60k triangles: 781 -> 710 us; one FMA per plane 2 % and
     // compares with set bits 3 % slower). Empty slots hold inverted boxes
     // (qlo = 255, qhi = 0) that no ray enters; one accepted through rounding is a leaf of zero
