@@ -812,6 +812,13 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
     }
     k_last_passes<<<1, kLast, 0, st>>>(cl[cur], state + cur, N, width, root, &es->err);
     LMGPU_CUDA(cudaGetLastError());
+    // Non-finite input is refused here at the latest: from the allocations below on, the tree that the
+    // outputs may still hold is overwritten. The wait replaces the one for the root at the end.
+    RootInfo hr{};
+    LMGPU_CUDA(cudaMemcpyAsync(&hr, root, sizeof(hr), cudaMemcpyDeviceToHost, st));
+    LMGPU_CUDA(cudaMemcpyAsync(&herr, &es->err, 4, cudaMemcpyDeviceToHost, st));
+    LMGPU_CUDA(cudaStreamSynchronize(st));
+    check();
 
     // emission, four levels between two reads of how many nodes there are
     const int32_t cap = int32_t(std::max<int64_t>(n, 1));  // wide nodes never exceed the triangles
@@ -838,9 +845,6 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
     } while (!empty(levels));
     while (levels > 0 && empty(levels - 1)) levels--;
     if (int64_t(h.tri_count) != n) throw Error(LMGPU_ERR_INTERNAL, "accel build: internal error (triangle count)");
-    RootInfo hr{};
-    LMGPU_CUDA(cudaMemcpyAsync(&hr, root, sizeof(hr), cudaMemcpyDeviceToHost, st));
-    LMGPU_CUDA(cudaStreamSynchronize(st));
     const double dx = double(hr.hi[0]) - hr.lo[0], dy = double(hr.hi[1]) - hr.lo[1], dz = double(hr.hi[2]) - hr.lo[2];
     const double ra = 2.0 * (dx * dy + dy * dz + dz * dx);
     sah_cost = ra > 0 ? double(hr.cost) / ra : 0.0;
