@@ -418,11 +418,16 @@ __global__ void __launch_bounds__(kLast) k_last_passes(const int32_t* __restrict
 
 // ---- emission ------------------------------------------------------------------------------
 
-// Counters of the emission, one host read for all of them.
-struct EmitState {
+// Counters of the emission, one host read for all of them. `now` is copied to the ring after every
+// level, so that the error word a level reads is the same in all of its threads.
+struct LevelEnd {
+    int32_t wide_count;
     int err;
-    int32_t wide_count, tri_count;
-    int32_t level[8];  // ring: level l holds the wide nodes [level[l & 7], level[(l + 1) & 7])
+};
+struct EmitState {
+    LevelEnd now;
+    int32_t tri_count;
+    LevelEnd level[8];  // ring: level l holds the wide nodes [level[l & 7], level[(l + 1) & 7])
 };
 
 struct Emit {
@@ -457,9 +462,13 @@ __global__ void __launch_bounds__(kEmitBlock) k_emit(Emit E, int level) {
     const Nodes& N = E.N;
     const int lane = int(threadIdx.x & 31u), s = lane & 7;
     const unsigned gm = 0xffu << (lane & 24);
-    const int32_t w1 = E.st->level[(level + 1) & 7], root = E.root->root;
+    const LevelEnd end = E.st->level[(level + 1) & 7];
+    // a node with an error has counted its children and not written them, and the host looks only after
+    // four levels (merged boxes whose area overflows get here)
+    if (end.err) return;
+    const int32_t w1 = end.wide_count, root = E.root->root;
     auto from = [&](auto v, int src) { return __shfl_sync(gm, v, src, 8); };
-    for (int32_t w = E.st->level[level & 7] + (int32_t(blockIdx.x) * kEmitBlock + int32_t(threadIdx.x)) / 8; w < w1;
+    for (int32_t w = E.st->level[level & 7].wide_count + (int32_t(blockIdx.x) * kEmitBlock + int32_t(threadIdx.x)) / 8; w < w1;
          w += int32_t(gridDim.x) * (kEmitBlock / 8)) {
         const int32_t bin = E.q_bin[w];
         // the node's children (binary node ids), depth-first left before right: child i goes to lane i
@@ -500,7 +509,7 @@ __global__ void __launch_bounds__(kEmitBlock) k_emit(Emit E, int level) {
             }
         }
         if (bad) {  // the same in all lanes of the group
-            atomicOr(&E.st->err, kErrLayout);
+            atomicOr(&E.st->now.err, kErrLayout);
             continue;
         }
         // octant-ordered slots (bvh_build.cpp: greedy on dot(centroid - center, octant direction))
@@ -559,7 +568,7 @@ __global__ void __launch_bounds__(kEmitBlock) k_emit(Emit E, int level) {
             if (s == bi) placed = true;
         }
         if (bad) {
-            atomicOr(&E.st->err, kErrLayout);
+            atomicOr(&E.st->now.err, kErrLayout);
             continue;
         }
         // lane s takes over the child of slot s
@@ -583,13 +592,13 @@ __global__ void __launch_bounds__(kEmitBlock) k_emit(Emit E, int level) {
         off -= mine;
         int32_t child_base = 0, tri_base = 0;
         if (s == 0) {
-            child_base = nint ? atomicAdd(&E.st->wide_count, nint) : 0;
+            child_base = nint ? atomicAdd(&E.st->now.wide_count, nint) : 0;
             tri_base = ntri ? atomicAdd(&E.st->tri_count, ntri) : 0;
         }
         child_base = from(child_base, 0);
         tri_base = from(tri_base, 0);
         if (__any_sync(gm, child_base + nint > E.wide_cap || (is_leaf && (cnt < 1 || cnt > kMaxLeaf || off > 31)))) {
-            atomicOr(&E.st->err, kErrLayout);
+            atomicOr(&E.st->now.err, kErrLayout);
             continue;
         }
         uint32_t meta = 0u;
@@ -664,11 +673,11 @@ __global__ void __launch_bounds__(kEmitBlock) k_emit(Emit E, int level) {
             quantized = quantized && ok;
         }
         if (__any_sync(gm, bad)) {
-            atomicOr(&E.st->err, kErrLayout);
+            atomicOr(&E.st->now.err, kErrLayout);
             continue;
         }
         if (!quantized) {  // the same in all lanes of the group
-            atomicOr(&E.st->err, kErrQuantize);
+            atomicOr(&E.st->now.err, kErrQuantize);
             continue;
         }
         // four slots' bytes per word: lanes 0-3 the first, 4-7 the second
@@ -706,10 +715,10 @@ __global__ void __launch_bounds__(kEmitBlock) k_emit(Emit E, int level) {
 // Level 0: the root's wide node.
 __global__ void k_emit_start(Emit E) {
     E.q_bin[0] = E.root->root;
-    E.st->wide_count = 1;
+    E.st->now.wide_count = 1;
     E.st->tri_count = 0;
-    E.st->level[0] = 0;
-    E.st->level[1] = 1;
+    E.st->level[0] = LevelEnd{0, 0};
+    E.st->level[1] = LevelEnd{1, 0};
 }
 
 int grid_of(int64_t n) { return int(std::min<int64_t>((n + kBlock - 1) / kBlock, int64_t(1) << 20)); }
@@ -772,7 +781,7 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
     LMGPU_CUDA(cudaMemsetAsync(cb + 3, 0, 12, st));
     LMGPU_CUDA(cudaMemsetAsync(es, 0, sizeof(EmitState), st));
     const int g = grid_of(n);
-    k_prep<<<g, kBlock, 0, st>>>(P, n, tlo, thi, cen, cb, &es->err);
+    k_prep<<<g, kBlock, 0, st>>>(P, n, tlo, thi, cen, cb, &es->now.err);
     k_morton<<<g, kBlock, 0, st>>>(cen, n, cb, keys[0], vals[0]);
     LMGPU_CUDA(cudaGetLastError());
     cub::DoubleBuffer<uint32_t> dk(keys[0], keys[1]);
@@ -802,7 +811,7 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
         }
         PlocState h{};
         LMGPU_CUDA(cudaMemcpyAsync(&h, state + cur, sizeof(h), cudaMemcpyDeviceToHost, st));
-        LMGPU_CUDA(cudaMemcpyAsync(&herr, &es->err, 4, cudaMemcpyDeviceToHost, st));
+        LMGPU_CUDA(cudaMemcpyAsync(&herr, &es->now.err, 4, cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaStreamSynchronize(st));
         check();
         if (h.m < 1 || h.m >= m || h.next_id - int32_t(n) != int32_t(n) - h.m)
@@ -810,13 +819,13 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
         m = h.m;
         if (++iters > 100000) throw Error(LMGPU_ERR_INTERNAL, "accel build: clustering did not converge");
     }
-    k_last_passes<<<1, kLast, 0, st>>>(cl[cur], state + cur, N, width, root, &es->err);
+    k_last_passes<<<1, kLast, 0, st>>>(cl[cur], state + cur, N, width, root, &es->now.err);
     LMGPU_CUDA(cudaGetLastError());
     // Non-finite input is refused here at the latest: from the allocations below on, the tree that the
     // outputs may still hold is overwritten. The wait replaces the one for the root at the end.
     RootInfo hr{};
     LMGPU_CUDA(cudaMemcpyAsync(&hr, root, sizeof(hr), cudaMemcpyDeviceToHost, st));
-    LMGPU_CUDA(cudaMemcpyAsync(&herr, &es->err, 4, cudaMemcpyDeviceToHost, st));
+    LMGPU_CUDA(cudaMemcpyAsync(&herr, &es->now.err, 4, cudaMemcpyDeviceToHost, st));
     LMGPU_CUDA(cudaStreamSynchronize(st));
     check();
 
@@ -831,16 +840,16 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
     EmitState h{};
     int32_t levels = 0;
     const int emit_grid = int(std::min<int64_t>((n + kEmitBlock / 8 - 1) / (kEmitBlock / 8), int64_t(current_device().num_sms) * 16));
-    auto empty = [&](int32_t l) { return h.level[l & 7] == h.level[(l + 1) & 7]; };
+    auto empty = [&](int32_t l) { return h.level[l & 7].wide_count == h.level[(l + 1) & 7].wide_count; };
     do {
         for (int k = 0; k < 4; k++, levels++) {
             k_emit<<<emit_grid, kEmitBlock, 0, st>>>(E, levels);
             LMGPU_CUDA(cudaGetLastError());
-            LMGPU_CUDA(cudaMemcpyAsync(&es->level[(levels + 2) & 7], &es->wide_count, 4, cudaMemcpyDeviceToDevice, st));
+            LMGPU_CUDA(cudaMemcpyAsync(&es->level[(levels + 2) & 7], &es->now, sizeof(LevelEnd), cudaMemcpyDeviceToDevice, st));
         }
         LMGPU_CUDA(cudaMemcpyAsync(&h, es, sizeof(h), cudaMemcpyDeviceToHost, st));
         LMGPU_CUDA(cudaStreamSynchronize(st));
-        herr = h.err;
+        herr = h.now.err;
         check();
     } while (!empty(levels));
     while (levels > 0 && empty(levels - 1)) levels--;
@@ -848,7 +857,7 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
     const double dx = double(hr.hi[0]) - hr.lo[0], dy = double(hr.hi[1]) - hr.lo[1], dz = double(hr.hi[2]) - hr.lo[2];
     const double ra = 2.0 * (dx * dy + dy * dz + dz * dx);
     sah_cost = ra > 0 ? double(hr.cost) / ra : 0.0;
-    num_nodes = h.wide_count;
+    num_nodes = h.now.wide_count;
     depth = levels;
 }
 
