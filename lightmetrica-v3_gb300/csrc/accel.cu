@@ -348,17 +348,15 @@ int lmgpu_accel_build_ex(lmgpu_accel* accel, const float* tri_p, int64_t num_tri
         if (builder == LMGPU_BUILDER_GPU_PLOC) {
             cudaStream_t st;
             LMGPU_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-            int64_t nn = 0;
             int32_t depth = 0;
             double sah = 0;
             try {
-                build_bvh8_gpu(tri_p, num_tris, accel->nodes, accel->tris, accel->tri_slot, nn, depth, sah, st);
+                build_bvh8_gpu(tri_p, num_tris, accel->nodes, accel->tris, accel->tri_slot, accel->num_nodes, depth, sah, st);
             } catch (...) {
                 cudaStreamDestroy(st);
                 throw;
             }
             cudaStreamDestroy(st);
-            accel->num_nodes = nn;
             accel->depth = depth;
             accel->sah_cost = sah;
         } else {

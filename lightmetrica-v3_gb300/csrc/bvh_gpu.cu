@@ -830,6 +830,7 @@ void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, 
     check();
 
     // emission, four levels between two reads of how many nodes there are
+    num_nodes = 0;  // until it is done the outputs hold no tree
     const int32_t cap = int32_t(std::max<int64_t>(n, 1));  // wide nodes never exceed the triangles
     nodes.alloc(size_t(cap) * 80);
     tris.alloc(size_t(n) * 48);

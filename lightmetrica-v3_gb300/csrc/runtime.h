@@ -95,7 +95,8 @@ struct DevBuf {
 };
 
 // GPU builder of the 8-wide tree (bvh_gpu.cu): device buffers in the layout of bvh_build.h, plus
-// the flattened-index -> record map. Synchronous on `st`.
+// the flattened-index -> record map. Synchronous on `st`. On an error num_nodes tells what the buffers
+// hold: unchanged, what they held before; 0, no tree.
 void build_bvh8_gpu(const float* tri_p, int64_t n, DevBuf& nodes, DevBuf& tris, DevBuf& tri_slot, int64_t& num_nodes,
                     int32_t& depth, double& sah_cost, cudaStream_t st);
 

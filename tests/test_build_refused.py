@@ -56,3 +56,20 @@ def test_areas_beyond_the_float_range(lm, a, b):
     fresh = lm.load_accel("fresh", "sahbvh", builder="sah")
     fresh.build_triangles(_soup(2000, 4))
     assert acc.intersect_batch(rays).tobytes() == fresh.intersect_batch(rays).tobytes()
+
+
+@pytest.mark.parametrize("built", [9, 5000])  # larger and smaller buffers than the refused mesh takes
+def test_rebuild_refused_late(lm, built):
+    """An emission that fails has overwritten the accel's tree: queries are refused until the next build."""
+    from lightmetrica._native import LmGpuError
+    acc = lm.load_accel("acc", "sahbvh", builder="ploc")
+    acc.build_triangles(_soup(built, 3))
+    with pytest.raises(LmGpuError, match="wide node layout"):
+        acc.build_triangles(_overflowing(6, 200))
+    rays = _rays(5000, 5)
+    with pytest.raises(LmGpuError, match="not built"):
+        acc.intersect_batch(rays)
+    acc.build_triangles(_soup(2000, 4))
+    fresh = lm.load_accel("fresh", "sahbvh", builder="sah")
+    fresh.build_triangles(_soup(2000, 4))
+    assert acc.intersect_batch(rays).tobytes() == fresh.intersect_batch(rays).tobytes()
