@@ -185,6 +185,11 @@ struct Trav {
 };
 constexpr uint32_t kNoNode = 0xffffffffu;
 
+// Lanes per ray and rays per warp of the cooperative traversal (see coop_loop), and the lanes of lane
+// `lane`'s group.
+constexpr int kCoopLanes = 8, kCoopRays = 32 / kCoopLanes;
+__device__ __forceinline__ unsigned group_mask(unsigned lane) { return 0xffu << (lane & unsigned(32 - kCoopLanes)); }
+
 __device__ inline void trav_set_ray(Trav& s, f3 o, f3 d) {
     s.o = o;
     s.d = d;
@@ -330,10 +335,12 @@ __device__ __forceinline__ void trav_enter_instance(const Bvh8& bvh, Trav& s, co
 
 // Chooses s.node: the nearest of the entered inner children `inner` (slots of the node whose
 // children start at `base`, with child mask `imask`), else of the sibling group on top of the
-// stack, else kNoNode. False on a stack overflow. `write`: this lane stores the stack entry.
-template <bool kTwoLevel>
+// stack, else kNoNode. False on a stack overflow. kGroup: all lanes of a cooperative group call this on
+// the same ray and stack column; the first of them stores.
+template <bool kTwoLevel, bool kGroup = false>
 __device__ __forceinline__ bool trav_next(const Bvh8& bvh, Trav& s, uint32_t base, uint32_t imask, uint32_t inner, uint2* stk,
-                                          int stride, bool write = true) {
+                                          int stride) {
+    const unsigned lane = threadIdx.x & 31u;
     if (inner == 0u) {
         if (kTwoLevel && s.sp == s.inst_sp) {  // the instance is done: back to the world ray
             trav_set_ray(s, s.wo, s.wd);
@@ -346,6 +353,8 @@ __device__ __forceinline__ bool trav_next(const Bvh8& bvh, Trav& s, uint32_t bas
         }
         s.sp--;
         const uint2 g = stk[s.sp * stride];
+        // what is left of the entry goes back to the same place: not before the whole group has read it
+        if (kGroup) __syncwarp(group_mask(lane));
         base = g.x;
         imask = g.y >> 8;
         inner = g.y & 0xffu;
@@ -361,7 +370,7 @@ __device__ __forceinline__ bool trav_next(const Bvh8& bvh, Trav& s, uint32_t bas
     inner ^= first;
     if (inner != 0u) {
         if (s.sp >= bvh.depth) return false;
-        if (write) stk[s.sp * stride] = make_uint2(base, (imask << 8) | inner);
+        if (!kGroup || lane % kCoopLanes == 0u) stk[s.sp * stride] = make_uint2(base, (imask << 8) | inner);
         s.sp++;
     }
     return true;
@@ -469,8 +478,6 @@ __device__ __forceinline__ void trace_end(const Fetch& f) {
 // longest rays take 100-200 steps of about 0.6 us, so a launch's last rays cost 100 us and more
 // whatever its size: 16k rays into a soup of 60k triangles 114 -> 89 us, 200k 195 -> 179 us, the
 // light-traced frame (18 trace launches) 3.68 -> 3.31 ms with the smaller blocks of its kernels.
-constexpr int kCoopLanes = 8, kCoopRays = 32 / kCoopLanes;
-
 // Tests the triangles s.tri_mask of each group's ray (same in the group's lanes); any hit: true in
 // the lanes of a group whose ray hits one. Called by full warps; groups without a ray: mask 0.
 template <bool kAnyHit, bool kTwoLevel>
@@ -580,8 +587,7 @@ __device__ __forceinline__ void coop_loop(const Bvh8& bvh, Trav& s, bool live, i
         s.tri_mask = tm;
         if (coop_tris<kAnyHit, kTwoLevel>(bvh, s)) done = true;
         if (test && !done) {
-            // every lane follows the same path; one of them writes the stack
-            if (!trav_next<kTwoLevel>(bvh, s, w1.x, imask, hit & imask, stk, stride, sub == 0u)) {
+            if (!trav_next<kTwoLevel, true>(bvh, s, w1.x, imask, hit & imask, stk, stride)) {
                 *lerr = 1;
                 done = true;
             }
