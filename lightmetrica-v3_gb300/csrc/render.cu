@@ -3401,6 +3401,11 @@ int lmgpu_render_pt_noalloc(lmgpu_scene* s, float* d_film, int32_t w, int32_t h,
 // ---------------------------------------------------------------------------------------------
 // Shared wavefront over many jobs (lmgpu_batch_*)
 
+namespace lmgpu {
+constexpr int kChunkIters = 8;      // even: the queue parity is the same at every chunk boundary
+constexpr int kMaxChunkIters = 16;  // longest chunk (one job whose paths all start at once); even
+}  // namespace lmgpu
+
 struct lmgpu_batch {
     int64_t cap = 0;
     lmgpu::DevBuf q_o[2], q_d[2], q_thr[2], q_nrm[2], q_ids[2], q_job[2], hits, s_o, s_d, s_c, s_job;
@@ -3424,17 +3429,18 @@ struct lmgpu_batch {
     uint32_t passes = 0;
     bool table_dirty = false;
     int32_t max_depth = 1;
-    // Captured chunk of iterations: [0] plain, [1] with the kernels' time stamps, [2] and [3] the same for
-    // tables with an instanced scene, whose two-level traversal and deeper stacks would slow plain ones
-    // (1080p frame at 16 spp after an instanced scene 32.3 ms, 25.0 with its own chunk; a plain and an
-    // instanced 64x64 preview in turn 580 us each, 379).
+    // Captured chunks of iterations, made when first run and kept until a device table moves. One each
+    // for what a program may change from call to call: time stamps or none; tables without or with an
+    // instanced scene, whose two-level traversal and deeper stacks would slow plain ones (1080p frame at
+    // 16 spp after an instanced scene 32.3 ms, 25.0 with its own chunk; a plain and an instanced 64x64
+    // preview in turn 580 us each, 379); pixel or image mode; and the iterations, which follow the path
+    // length of one job (64x64 previews of 9 and 13 vertices in turn 491 and 617 us where they share a
+    // place, 292 and 385 so, as alone). Sixteen of them took 8 MB of device memory in all.
     struct GraphSlot {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         int32_t depth = 0;
         int refill = -1, shade = -1, first_pass = -1, specialize = -1;
-        bool two_level = false, image = false;
-        int iters = 0;
         bool single = false;      // captured for a one-job table
         uint32_t feat = 0;        // that job's scene features (the shade kernel specialised for them)
         lmgpu::Bvh8 bvh{};        // that job's tree and films, passed by value to the trace kernels
@@ -3449,7 +3455,7 @@ struct lmgpu_batch {
             ext_nodes.clear();
             sh_nodes.clear();
         }
-    } slot[4];
+    } slot[2][2][2][lmgpu::kMaxChunkIters / 2];
     int32_t stack_depth[2] = {1, 1};  // the deepest tree yet of tables without and with instances
     int refill = 0, shade_minblocks = 3, first_pass = 1, specialize = 1;
     bool two_level = false;  // some job's scene is instanced
@@ -3459,8 +3465,15 @@ struct lmgpu_batch {
     double kms[4] = {0, 0, 0, 0};  // extend, shade, shadow, plan + generate
     int64_t iters_run = 0;
     double elapsed_ms = 0;
+    template <typename F>
+    void each_slot(F f) {
+        for (auto& a : slot)
+            for (auto& b : a)
+                for (auto& c : b)
+                    for (GraphSlot& g : c) f(g);
+    }
     ~lmgpu_batch() {
-        for (GraphSlot& g : slot) g.clear();
+        each_slot([](GraphSlot& g) { g.clear(); });
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
     }
@@ -3468,9 +3481,6 @@ struct lmgpu_batch {
 
 namespace lmgpu {
 namespace {
-
-constexpr int kChunkIters = 8;      // even: the queue parity is the same at every chunk boundary
-constexpr int kMaxChunkIters = 16;  // longest chunk (one job whose paths all start at once)
 
 // Control words. The planner indexes the first 32 as int64 (its comment); the rest are counters, each
 // written only by launches that none of its readers runs beside.
@@ -3660,18 +3670,16 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc, int iters) {
     b->shade_minblocks = tuning().shade_minblocks;
     b->first_pass = tuning().batch_first_pass;
     b->specialize = tuning().shade_specialize;
-    if (realloc)
-        for (auto& old : b->slot) old.clear();
-    auto& g = b->slot[(b->timed ? 1 : 0) + (b->two_level ? 2 : 0)];
+    if (realloc) b->each_slot([](lmgpu_batch::GraphSlot& old) { old.clear(); });
+    auto& g = b->slot[b->timed][b->two_level][b->image][iters / 2 - 1];
     // stacks only grow within a kind of table, so that scenes of other depths share its chunk
     int32_t& depth = b->stack_depth[b->two_level ? 1 : 0];
     b->max_depth = depth = std::max(depth, b->max_depth);
     const bool single = b->host_jobs.size() == 1;
     const uint32_t feat = table_features(b);
     const bool same_shape = g.exec && g.depth == b->max_depth && g.refill == b->refill && g.shade == b->shade_minblocks &&
-                            g.two_level == b->two_level && g.first_pass == b->first_pass && g.single == single &&
-                            g.feat == feat && g.specialize == b->specialize && g.iters == iters &&
-                            g.image == b->image;
+                            g.first_pass == b->first_pass && g.single == single && g.feat == feat &&
+                            g.specialize == b->specialize;
     auto same_job = [&] {
         const JobDev& J = b->host_jobs[0];
         return std::memcmp(&g.bvh, &J.S.bvh, sizeof(Bvh8)) == 0 && g.film == J.film && g.film_odd == J.film_odd;
@@ -3747,13 +3755,10 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc, int iters) {
     g.sh_nodes = std::move(sh_nodes);
     g.depth = b->max_depth;
     g.refill = b->refill;
-    g.two_level = b->two_level;
     g.first_pass = b->first_pass;
     g.shade = b->shade_minblocks;
     g.specialize = b->specialize;
     g.single = single;
-    g.iters = iters;
-    g.image = b->image;
     g.feat = feat;
     if (single) {
         g.bvh = b->host_jobs[0].S.bvh;
