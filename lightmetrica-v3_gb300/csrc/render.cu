@@ -3701,6 +3701,8 @@ cudaGraphExec_t ensure_graph(lmgpu_batch* b, bool realloc, int iters) {
             kp.kernelParams = args.data();
             LMGPU_CUDA(cudaGraphExecKernelNodeSetParams(g.exec, node, &kp));
         };
+        g.bvh = Bvh8{};  // no job's until every launch is set: a failure in between leaves launches of both
+        g.film = g.film_odd = nullptr;
         for (auto node : g.ext_nodes) set(node, {{0, &tb}}, 13);
         for (auto node : g.sh_nodes) set(node, {{0, &tb}, {3, &film}, {11, &film_odd}}, 12);
         g.bvh = J.S.bvh;
