@@ -382,9 +382,8 @@ def run_gpu(args) -> None:
                "sample": f"{W_PX}x{H_PX} at 1 spp ({W_PX * H_PX} paths, {crays} rays, {csec:.1f} s)",
                "build_seconds": S.build_seconds}
 
-    # kernels per step: every chunk of the shared wavefront launches extend, shade, shadow, plan and
-    # generate once per bounce iteration; one film resolve per render
-    # per iteration generate, extend, shade and shadow; the film scaling
+    # kernels per step: every bounce iteration of the shared wavefront launches generate, extend, shade
+    # and shadow (one job: no planner); one film scaling per render
     launches_per_step = 4 * tot["ext_launches"] / max(1, args.steps) + 1
     if rank == 0:
         out = {

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(Bvh8 bvh, const flo
         if (threadIdx.x == 0) s_fetch = 0;
         __syncthreads();
         fetch_loop<kAnyHit, false, kTwoLevel>(
-            int(count), int(blockDim.x / 32), Fetch{&s_fetch, {nullptr, nullptr}, refill, nullptr, nullptr}, stk, stride, &lerr,
+            int(count), int(blockDim.x / 32), Fetch{&s_fetch, nullptr, refill, nullptr, nullptr}, stk, stride, &lerr,
             [&](int k, Trav& s) {
                 const int64_t i = ray_of(k);
                 const float4 a = rays[2 * i], b = rays[2 * i + 1];
@@ -239,9 +239,13 @@ void launch_trace(const lmgpu_accel* a, const void* d_rays, int64_t n, void* d_h
     const Bvh8 b = device_view(a);
     const size_t smem = trace_smem(a);
     const bool two = a->num_instances > 0, refine = !d_occ && !two && a->tri_slot.p;
-    // Batches of at most one ray per resident lane refine their hits in the trace launch: 2^10 rays
-    // 66.7 -> 60.7 us, 2^17 178 -> 174. Larger ones in a launch of their own: with the refinement's
-    // code the trace kernel takes 79 instead of 72 registers (2^20 rays 616 -> 644 us).
+    // Batches of at most 1,024 rays per SM (768 lanes are in flight on one, at 79 registers and at the 80
+    // with the refinement's code) refine their hits in the trace launch, larger ones in a launch of their
+    // own, whose warps hold hits only. The launch saved is worth 3-5 us. Separate and fused, in us,
+    // diffuse bounces in a soup of 60k triangles: 2^10 rays 56.4 and 50.3, 2^14 83.6 and 79.3, 2^17 137
+    // and 139, 155,648 (the line on 152 SMs) 148 and 151, 2^18 207 and 210, 2^19 349 and 360, 2^20 614
+    // and 641; camera rays 2^14 76.9 and 73.4, 155,648 106 and 105, 2^18 127 and 125, 2^19 191 and 196;
+    // 1,009 triangles 155,648 45.7 and 42.3, 2^18 61.9 and 60.2, 2^19 100.8 and 105.
     const bool fused = refine && tuning().trace_refill > 0 && n <= int64_t(current_device().num_sms) * 1024;
     auto run = [&](auto kernel) {
         // Rays per group: 32, or fewer when the batch has fewer rays than the chip has lanes, so that

@@ -209,7 +209,7 @@ __device__ inline void trav_init(Trav& s, f3 o, f3 d, float tmin, float tmax) {
     // -0 for a zero: the box comparison is the sign of far * kWiden - near, and a hit at t = -0 (a ray
     // that starts on a surface) as the far side against +0 gives -0, a miss of boxes with hits at the
     // same t and a smaller index; against -0 it gives +0.
-    s.tmin = tmin == 0.0f ? -0.0f : tmin;
+    s.tmin = -(0.0f - tmin);
     s.best = TraceHit{tmax, 0.f, 0.f, -1};
     s.sp = 0;
     s.node = 0;
@@ -400,8 +400,8 @@ __device__ __forceinline__ bool trav_step(const Bvh8& bvh, Trav& s, uint2* stk, 
     return s.node == kNoNode;
 }
 
-// trav_step's node part alone, for single-level trees (after the triangle postponing of Ylitie et
-// al., HPG 2017): visits s.node and only records the triangles of the entered leaf children. A ray
+// trav_step's node part alone, for single-level trees (after the speculative traversal of Aila & Laine,
+// HPG 2009): visits s.node and only records the triangles of the entered leaf children. A ray
 // may visit further nodes while one node's triangles wait (not while two nodes' do), so a warp can
 // choose the step that most of its lanes can take; a visit before a nearer hit is known may enter
 // more nodes, the result is the same. Returns true when no node and no triangle is left.
@@ -443,21 +443,20 @@ __device__ inline unsigned long long globaltimer_ns() {
 }
 
 // Dynamic ray fetch for the persistent trace kernels: `self` hands out queue entries (zero at
-// launch). The launch zeroes the counters in `reset` (where set) at its start, for kernels that run
+// launch). The launch zeroes the counter `reset` (where set) at its start, for a kernel that runs
 // after it and that no kernel in flight uses. refill: see Tuning. With `stamp`, the launch writes its
 // start and end times there ([0], [1], in ns); `done` counts its finished blocks (zero between
 // launches).
 struct Fetch {
     int* self;
-    int* reset[2];
+    int* reset;
     int refill;
     unsigned long long* stamp;
     int* done;
 };
 __device__ __forceinline__ void trace_begin(const Fetch& f) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    if (f.reset[0]) *f.reset[0] = 0;
-    if (f.reset[1]) *f.reset[1] = 0;
+    if (f.reset) *f.reset = 0;
     if (f.stamp) f.stamp[0] = globaltimer_ns();
 }
 // Called by all threads of the block at the launch's end.
@@ -664,7 +663,7 @@ __device__ __forceinline__ void fetch_loop(int n, int warps, const Fetch& f, uin
                         done = done || (s.tri_mask == 0u && s.node == kNoNode);
                     }
                 } else {
-                    if (active && !done && s.tri_mask2 == 0u && s.node != kNoNode) done = trav_node(B, s, stk, stride, lerr);
+                    if (active && s.tri_mask2 == 0u && s.node != kNoNode) done = trav_node(B, s, stk, stride, lerr);
                 }
             }
             if (done) active = false;

@@ -2748,7 +2748,7 @@ void render_pt_waves(lmgpu_scene* s, lmgpu_film* f, const lmgpu_pt_params* prm, 
         // [0],[1] extension queues, [2] shadow queue, [3] error, [4],[5] extension / shadow ray fetch
         int* cnt = ws.counters.as<int>();
         const int refill = tuning().trace_refill;
-        const Fetch f_ext{cnt + 4, {cnt + 5, nullptr}, refill, nullptr, nullptr}, f_sh{cnt + 5, {cnt + 4, nullptr}, refill, nullptr, nullptr};
+        const Fetch f_ext{cnt + 4, cnt + 5, refill, nullptr, nullptr}, f_sh{cnt + 5, cnt + 4, refill, nullptr, nullptr};
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(ws.counters.as<char>() + 32);
         float* film = f->sum.as<float>();
         const Bvh8 bvh = s->dev.bvh;
@@ -3010,8 +3010,8 @@ int lmgpu_render_lt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_lt_params* prm, v
                 int *sc = cnt + (it & 1 ? 2 : 6), *sc_next = cnt + (it & 1 ? 6 : 2);
                 IterStamps* T = timed ? ws.stamps.as<IterStamps>() + stamped : nullptr;
                 stamped++;
-                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, timed ? T->ext : nullptr, cnt + 48};
-                const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, timed ? T->shadow : nullptr, cnt + 49};
+                const Fetch f_ext{cnt + 4, cnt + (1 - cur), refill, timed ? T->ext : nullptr, cnt + 48};
+                const Fetch f_sh{cnt + 5, nullptr, refill, timed ? T->shadow : nullptr, cnt + 49};
                 ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
                 n_ext++;
@@ -3177,7 +3177,7 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
                 // the shade kernel zeroes the fetch counter for the next bounce's launch
                 IterStamps* T = timed ? ws.stamps.as<IterStamps>() + stamped : nullptr;
                 stamped++;
-                const Fetch f_ext{cnt + 4, {cnt + (1 - cur), nullptr}, refill, timed ? T->ext : nullptr, cnt + 48};
+                const Fetch f_ext{cnt + 4, cnt + (1 - cur), refill, timed ? T->ext : nullptr, cnt + 48};
                 ext_k<<<g_ext, kTrace, tsmem, st>>>(bvh, q[cur].o, q[cur].d, cnt + cur, ws.hits.as<float4>(), rays, cnt + 3, nullptr,
                                                     0, nullptr, f_ext, nullptr, nullptr);
                 n_ext++;
@@ -3189,7 +3189,7 @@ int lmgpu_render_bdpt(lmgpu_scene* s, lmgpu_film* f, const lmgpu_bdpt_params* pr
             // the connections' own entry: `shade` the strategy list's start, `shadow` the visibility rays
             IterStamps* T = timed ? ws.stamps.as<IterStamps>() + stamped : nullptr;
             stamped++;
-            const Fetch f_sh{cnt + 5, {nullptr, nullptr}, refill, timed ? T->shadow : nullptr, cnt + 49};
+            const Fetch f_sh{cnt + 5, nullptr, refill, timed ? T->shadow : nullptr, cnt + 49};
             LMGPU_CUDA(cudaMemsetAsync(cnt + 6, 0, 4, st));
             k_bd_items<<<int(std::min<int64_t>(g_items, (n + kBlock - 1) / kBlock)), kBlock, 0, st>>>(
                 R, n, prm->min_verts, mv, ws.bd_items.as<uint2>(), cnt + 6, icap, cnt + 3, timed ? &T->shade : nullptr);
@@ -3314,7 +3314,7 @@ int lmgpu_render_pt_noalloc(lmgpu_scene* s, float* d_film, int32_t w, int32_t h,
         // [0],[1] extension queues, [2] shadow queue, [3] error, [4],[5] extension / shadow ray fetch
         int* cnt = reinterpret_cast<int*>(base);
         const int refill = tuning().trace_refill;
-        const Fetch f_ext{cnt + 4, {cnt + 5, nullptr}, refill, nullptr, nullptr}, f_sh{cnt + 5, {cnt + 4, nullptr}, refill, nullptr, nullptr};
+        const Fetch f_ext{cnt + 4, cnt + 5, refill, nullptr, nullptr}, f_sh{cnt + 5, cnt + 4, refill, nullptr, nullptr};
         unsigned long long* rays = reinterpret_cast<unsigned long long*>(base + 32);
         unsigned long long* sums = reinterpret_cast<unsigned long long*>(base + 64);
         char* p = base + kNoallocCounters;
@@ -3493,7 +3493,6 @@ struct Ctl {
     int64_t seen, active, allocs;                      // [20]..[22]
     int shadow_odd, done[2], pad3;                     // finished blocks of the timed trace launches
     int64_t started_odd;
-    unsigned long long end;                            // start of the launch after the last iteration
     IterStamps it[kMaxChunkIters];
 };
 static_assert(offsetof(Ctl, survivors) == 48 && offsetof(Ctl, rays) == 64 && offsetof(Ctl, fetch) == 144 && offsetof(Ctl, seen) == 160,
@@ -3523,10 +3522,7 @@ void grow_upload(DevBuf& buf, size_t& cap, size_t& done, const std::vector<T>& v
 }
 
 // paths in flight (the queue the next iteration starts from) plus paths not started yet
-__global__ void k_wf_left(Ctl* c, int cur, int timed) {
-    c->left = int64_t(c->survivors[cur]) + (c->total - c->started);
-    if (timed) c->end = globaltimer_ns();
-}
+__global__ void k_wf_left(Ctl* c, int cur) { c->left = int64_t(c->survivors[cur]) + (c->total - c->started); }
 
 __global__ void k_wf_set_total(int64_t* ctl, int64_t total, int64_t njobs) {
     ctl[1] = total;
@@ -3639,7 +3635,7 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent
                                         b->alloc.as<AllocEntry>(), b->first_pass, timed ? &T->gen : nullptr);
         gen_k<<<g_gen, kBlock, 0, st>>>(jobs, b->alloc.as<AllocEntry>(), ctl64(b), G, q[cur], sq, sc);
         ext_k<<<g_ext, kTrace, tsmem, st>>>(tb, q[cur].o, q[cur].d, &c->qn[cur], hits, &c->rays[0], &c->err, c->sums, 63, nullptr,
-                                            Fetch{&c->fetch[0], {&c->survivors[1 - cur], nullptr}, b->refill,
+                                            Fetch{&c->fetch[0], &c->survivors[1 - cur], b->refill,
                                                   timed ? T->ext : nullptr, &c->done[0]},
                                             single ? nullptr : jobs, single ? nullptr : q[cur].job);
         LMGPU_CUDA(cudaGetLastError());
@@ -3651,7 +3647,7 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent
         LMGPU_CUDA(cudaEventRecord(shaded, st));
         LMGPU_CUDA(cudaStreamWaitEvent(side, shaded, 0));
         sh_k<<<g_sh, kTrace, tsmem, side>>>(tb, sq, sc, sfilm, &c->rays[1], &c->err, c->sums, 63, nullptr,
-                                            Fetch{&c->fetch[1], {nullptr, nullptr}, b->refill, timed ? T->shadow : nullptr, &c->done[1]},
+                                            Fetch{&c->fetch[1], nullptr, b->refill, timed ? T->shadow : nullptr, &c->done[1]},
                                             single ? nullptr : jobs, single ? J0.film_odd : nullptr);
         LMGPU_CUDA(cudaGetLastError());
         sh_nodes.push_back(node_of(side));
@@ -3660,7 +3656,7 @@ void enqueue_chunk(lmgpu_batch* b, cudaStream_t st, cudaStream_t side, cudaEvent
         cur = 1 - cur;
     }
     // exact count of paths in flight or not started, for the host's end-of-chunk check
-    k_wf_left<<<1, 1, 0, st>>>(c, cur, timed ? 1 : 0);
+    k_wf_left<<<1, 1, 0, st>>>(c, cur);
 }
 
 // The executable graph for the current tuning, depth and timing; recaptured only when one of
