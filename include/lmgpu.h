@@ -98,7 +98,9 @@ int lmgpu_accel_build(lmgpu_accel* accel, const float* tri_p, int64_t num_tris);
  *  LMGPU_BUILDER_HOST_SAH -- binned SAH binary tree on the host threads, SAH-optimal 8-wide
  *                            collapse (lmgpu_accel_build's builder);
  *  LMGPU_BUILDER_GPU_PLOC -- on the GPU: Morton order, PLOC clustering into a binary tree, the same
- *                            SAH-optimal collapse and quantization. */
+ *                            SAH-optimal collapse and quantization.
+ * A GPU build that is refused for a non-finite vertex leaves the accel as it was. One that
+ * fails later (out of memory, boxes whose areas overflow) leaves it not built. */
 #define LMGPU_BUILDER_HOST_SAH 0
 #define LMGPU_BUILDER_GPU_PLOC 1
 int lmgpu_accel_build_ex(lmgpu_accel* accel, const float* tri_p, int64_t num_tris, int32_t builder);
